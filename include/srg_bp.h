@@ -453,13 +453,15 @@ int srg_forward_project_device(const srg_burst_desc *b, const float *refl,
  * Inputs: [nlines][ld] complex64 (device); nlines plays the reference's
  * <valid_lines>.  Outputs: [nlines/looksdn][na/looksac] complex64 (device).
  * Enqueued on `stream`.  FFTs in FP32 (the reference uses FFTW in single
- * precision, so results agree to FP32 rounding, not bit for bit): for lines
- * of 2,049-4,096 samples (nnn = 4,096) kernels of the library's own that
- * transform each line in shared memory (and, with looksdn = 1, form the
- * pairs there too, with no scratch but read-only tables), otherwise cuFFT.
- * The device's scratch (upsampled images) is shared by every call on it:
- * calls on the same device whose GPU work overlaps (other streams) race,
- * except those that form the pairs in shared memory. */
+ * precision, so results agree to FP32 rounding, not bit for bit), for lines of
+ * 33-65,536 samples by the library's own kernels, which make only the odd
+ * upsampled samples (the even ones are the input's, halved); otherwise cuFFT.
+ * The device's scratch (odd samples, 8 bytes per input sample of two images;
+ * with cuFFT the upsampled images) is shared by every call on it: calls on
+ * the same device whose GPU work overlaps (other streams) race, except those
+ * that form the pairs without scratch: looks of one line down (looksdn = 1)
+ * of lines of 33-4,096 samples.
+ */
 int srg_crossmul_device(const float *slc1, const float *slc2, long long ld, int na, int nlines,
                         int looksac, int looksdn, float scale, int mask, float *igram,
                         float *amp, void *stream);
