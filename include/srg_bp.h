@@ -487,10 +487,10 @@ int srg_range_replica(float samplefreq, float startfreq, float ramprate, float p
  * replica's 32,768-point spectrum, inverse FFT (unnormalised, as FFTW's), and
  * write the first nvalid = nsamps - npts samples of each line to `out`
  * ([nlines][ld_out] complex64, device; *nvalid_out receives nvalid).
- * Enqueued on `stream`.  Pulses of up to 4,096 samples: one fused kernel
- * forms those samples by overlap-save (8,192-point transforms in shared
- * memory; the same samples, the 32,768-point correlation never wrapping into
- * them); longer pulses: cuFFT.  FP32 throughout (the reference uses FFTW in
+ * Enqueued on `stream`.  Pulses of up to about 6,800 samples (whose lines
+ * take at most 20 segments): one fused kernel forms those samples by
+ * overlap-save (8,192-point transforms in shared memory; the same samples, the
+ * 32,768-point correlation never wrapping into them); longer pulses: cuFFT.  FP32 throughout (the reference uses FFTW in
  * single precision: results agree to FP32 rounding, not bit for bit).  The
  * device's scratch (the filter spectrum of the last pulse parameters, the
  * padded line blocks of the cuFFT path) is shared by every call on it: calls

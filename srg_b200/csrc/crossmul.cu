@@ -226,9 +226,11 @@ __device__ __forceinline__ void odd_samples(float2 (&v)[P::EPT], float2 *buf, in
 template <class P, bool STREAM>
 __device__ __forceinline__ void load_line(float2 (&v)[P::EPT], const float2 *__restrict__ x, int j,
                                           int na) {
+    x += j;
+    na -= j;
 #pragma unroll
     for (int i = 0; i < P::EPT; ++i) {
-        const int n = fftc::point_of<P>(j, i);
+        const int n = fftc::point_of<P>(i);
         v[i] = n < na ? (STREAM ? fftc::ld_stream(x + n) : __ldg(x + n)) : make_float2(0.f, 0.f);
     }
 }
@@ -264,11 +266,12 @@ odd_kernel(const __grid_constant__ OddArgs a, int nimg, long long ld, int na, in
         float2 v[P::EPT];
         load_line<P, !tables_in_smem<P>()>(v, a.in[k] + l * ld, j, mine ? na : 0);
         odd_samples<P>(v, buf, j, slot, LP == 1, tab);
-        float2 *out = a.odd[k] + l * na;
+        float2 *out = a.odd[k] + l * na + j;
+        const int nm = mine ? na - j : 0;
 #pragma unroll
         for (int i = 0; i < P::EPT; ++i) {
-            const int n = fftc::point_of<P>(j, i);
-            if (mine && n < na) out[n] = v[i];
+            const int n = fftc::point_of<P>(i);
+            if (n < nm) out[n] = v[i];
         }
         fftc::line_sync<P>(slot, LP == 1);  // the buffer's reads are done
     }
@@ -286,7 +289,7 @@ odd_kernel(const __grid_constant__ OddArgs a, int nimg, long long ld, int na, in
 // through distributed shared memory and writes C outputs per n.  So one
 // exchange per line, of the line's size, and two CTAs of different lines share
 // an SM.  Bound by instruction issue (53 % of the cycles) and the latency of
-// its loads: two images of 16,504 x 6,646 samples take 4.1 ms, where padding,
+// its loads: two images of 16,504 x 6,646 samples take 3.7 ms, where padding,
 // cuFFT's transforms of 32,768 and 65,536 points and the spread took 12.0; a
 // cluster of two with 16,384 points each, alone on its SMs, took 5.3.  The
 // grid is what the chip holds of clusters at once (with more, the last ones
@@ -344,11 +347,11 @@ odd_cluster_kernel(const __grid_constant__ OddArgs a, int nimg, long long ld, in
                 float2 b[16];
 #pragma unroll
                 for (int m = 0; m < 16; ++m) {
-                    const int n = j + (m0 + m) * P::T + c * P::M;
-                    b[m] = n < na ? fftc::ld_stream(x + n) : make_float2(0.f, 0.f);
+                    const int n = (m0 + m) * P::T + c * P::M;
+                    b[m] = n < na - j ? fftc::ld_stream(x + j + n) : make_float2(0.f, 0.f);
                 }
 #pragma unroll
-                for (int m = 0; m < 16; ++m) {  // point_of<P>(j, i) = j + (m0 + m) T
+                for (int m = 0; m < 16; ++m) {  // point_of<P>(i) = (m0 + m) T
                     const int i = (m0 + m) % P::GA * P::RA + (m0 + m) / P::GA;
                     v[i] = fftc::cadd(v[i], fftc::cmul(b[m], wc));
                 }
@@ -357,7 +360,7 @@ odd_cluster_kernel(const __grid_constant__ OddArgs a, int nimg, long long ld, in
         if (q) {
 #pragma unroll
             for (int i = 0; i < P::EPT; ++i)
-                v[i] = fftc::cmul(v[i], fftc::cmul(pre, turn[fftc::point_of<P>(0, i) / P::T]));
+                v[i] = fftc::cmul(v[i], fftc::cmul(pre, turn[fftc::point_of<P>(i) / P::T]));
         }
         // every CTA's reads of the line before are done
         if (item != blockIdx.x / C) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -365,8 +368,8 @@ odd_cluster_kernel(const __grid_constant__ OddArgs a, int nimg, long long ld, in
         __syncthreads();  // the buffer's reads are done
 #pragma unroll
         for (int i = 0; i < P::EPT; ++i) {
-            if (q) v[i] = fftc::cmul(v[i], fftc::cmulc(post, turn[fftc::point_of<P>(0, i) / P::T]));
-            buf[P::pad(fftc::point_of<P>(j, i))] = v[i];
+            if (q) v[i] = fftc::cmul(v[i], fftc::cmulc(post, turn[fftc::point_of<P>(i) / P::T]));
+            buf[P::pad(j + fftc::point_of<P>(i))] = v[i];
         }
         cl.sync();
         float2 *out = a.odd[k] + l * na;
@@ -395,7 +398,7 @@ odd_cluster_kernel(const __grid_constant__ OddArgs a, int nimg, long long ld, in
 // before, still in the thread's registers (its even samples are read again
 // from the input).  The images are read and the results written once.  Bound by
 // instruction issue and latency (two CTAs of 256 threads per SM, by their
-// registers): 32 images of 2,400 x 1,200 samples take 1.02 ms, 2.66 with
+// registers): 32 images of 2,400 x 1,200 samples take 0.96 ms, 2.66 with
 // self-sorting transforms of two lines per 512-thread CTA; of that, dealing
 // the steps evenly gave 12 %, reading the even samples in batches of four and
 // keeping each image's amplitudes another 10 %.
@@ -462,22 +465,23 @@ odd_stack_kernel(const __grid_constant__ StackPtrs p, int n, long long ld, int n
         const float2 *x1 = p.img[pair ? k - 1 : k] + row, *x2 = p.img[k] + row;
         float2 *ig = p.ig[pair ? k - 1 : 0] + l * nout, *am = p.am[pair ? k - 1 : 0] + l * nout;
         if constexpr (!ACROSS) {
+            const int nj = nm - j;
 #pragma unroll
             for (int h = 0; h < P::EPT; h += kBatch) {  // a batch of loads in flight
                 if (P::RA == P::EPT && h * P::T >= na) break;  // no column left
                 float2 e1[kBatch], e2[kBatch];
 #pragma unroll
                 for (int i = 0; i < kBatch; ++i) {
-                    const int c = fftc::point_of<P>(j, h + i);
+                    const int c = fftc::point_of<P>(h + i);
                     e1[i] = e2[i] = make_float2(0.f, 0.f);
-                    if (c < nm) {
-                        e1[i] = __ldg(x1 + c);
-                        e2[i] = __ldg(x2 + c);
+                    if (c < nj) {
+                        e1[i] = __ldg(x1 + j + c);
+                        e2[i] = __ldg(x2 + j + c);
                     }
                 }
 #pragma unroll
                 for (int i = 0; i < kBatch; ++i) {
-                    const int c = fftc::point_of<P>(j, h + i);
+                    const int c = fftc::point_of<P>(h + i);
                     const bool none = mask && empty_window(e2[i]);
                     const float2 f1 = make_float2(e1[i].x * even_scale, e1[i].y * even_scale);
                     const float2 f2 = make_float2(e2[i].x * even_scale, e2[i].y * even_scale);
@@ -489,9 +493,9 @@ odd_stack_kernel(const __grid_constant__ StackPtrs p, int n, long long ld, int n
                         fmaf(o1.y, o2.x, fmaf(-o1.x, o2.y, fmaf(f1.y, f2.x, -f1.x * f2.y))));
                     float2 a = make_float2(amp[h + i], p2);
                     if (none || (empty >> (h + i) & 1)) g = a = make_float2(0.f, 0.f);
-                    if (pair && c < nm) {
-                        ig[c] = g;
-                        am[c] = a;
+                    if (pair && c < nj) {
+                        ig[j + c] = g;
+                        am[j + c] = a;
                     }
                     amp[h + i] = p2;
                     empty = none ? empty | 1u << (h + i) : empty & ~(1u << (h + i));
@@ -505,7 +509,7 @@ odd_stack_kernel(const __grid_constant__ StackPtrs p, int n, long long ld, int n
             float p2[P::EPT];
 #pragma unroll
             for (int i = 0; i < P::EPT; ++i) {
-                const int c = fftc::point_of<P>(j, i);
+                const int c = j + fftc::point_of<P>(i);
                 const float2 o1 = prev[i], o2 = v[i];
                 float2 f1 = make_float2(0.f, 0.f), f2 = f1;
                 if (c < nm) {
@@ -531,7 +535,7 @@ odd_stack_kernel(const __grid_constant__ StackPtrs p, int n, long long ld, int n
             }
             fftc::line_sync<P>(slot, LP == 1);
 #pragma unroll
-            for (int i = 0; i < P::EPT; ++i) buf[P::pad(fftc::point_of<P>(j, i))].x = p2[i];
+            for (int i = 0; i < P::EPT; ++i) buf[P::pad(j + fftc::point_of<P>(i))].x = p2[i];
             fftc::line_sync<P>(slot, LP == 1);
 #pragma unroll
             for (int i = 0; i < P::EPT / 2; ++i) {

@@ -18,9 +18,10 @@
 // barriers and one more before the buffer is used again; the first pass reads
 // global memory and the last one leaves its results in registers.
 //
-// What bounds it: about as many cycles of the FP32 pipe (228 operations per
-// 16 points and pass: a 16-point DFT in 168, its twiddles in 60) as of the
-// shared-memory pipe (8 crossings of M points plus the twiddle tables).
+// What bounds it: instruction issue (per 16 points and pass about 208 FP32
+// operations, a 16-point DFT in 148 and its twiddles in 60, and 40 others) at
+// 55-65 % of the cycles: 16 warps per SM, by their 128 registers, do not cover
+// all of the latency of shared memory and barriers.
 //
 // Buffer layout: index i + i / EPT, which puts the accesses of every pass
 // (contiguous over threads, or EPT contiguous points per thread) on distinct
@@ -48,30 +49,30 @@ __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 
 // cos(2 pi q / 64), q = 0..16
-__host__ __device__ constexpr float cos64(int q) {
-    return q == 0    ? 1.f
-           : q == 1  ? 0.995184726672196886f
-           : q == 2  ? 0.980785280403230449f
-           : q == 3  ? 0.956940335732208865f
-           : q == 4  ? 0.923879532511286756f
-           : q == 5  ? 0.881921264348355030f
-           : q == 6  ? 0.831469612302545237f
-           : q == 7  ? 0.773010453362736961f
-           : q == 8  ? 0.707106781186547524f
-           : q == 9  ? 0.634393284163645498f
-           : q == 10 ? 0.555570233019602225f
-           : q == 11 ? 0.471396736825997649f
-           : q == 12 ? 0.382683432365089772f
-           : q == 13 ? 0.290284677254462368f
-           : q == 14 ? 0.195090322016128268f
-           : q == 15 ? 0.098017140329560602f
-                     : 0.f;
+__host__ __device__ constexpr double cos64(int q) {
+    return q == 0    ? 1.0
+           : q == 1  ? 0.995184726672196886
+           : q == 2  ? 0.980785280403230449
+           : q == 3  ? 0.956940335732208865
+           : q == 4  ? 0.923879532511286756
+           : q == 5  ? 0.881921264348355030
+           : q == 6  ? 0.831469612302545237
+           : q == 7  ? 0.773010453362736961
+           : q == 8  ? 0.707106781186547524
+           : q == 9  ? 0.634393284163645498
+           : q == 10 ? 0.555570233019602225
+           : q == 11 ? 0.471396736825997649
+           : q == 12 ? 0.382683432365089772
+           : q == 13 ? 0.290284677254462368
+           : q == 14 ? 0.195090322016128268
+           : q == 15 ? 0.098017140329560602
+                     : 0.0;
 }
-__host__ __device__ constexpr float cos_turn64(int q) {  // cos(2 pi q / 64), any q >= 0
+__host__ __device__ constexpr double cos_turn64(int q) {  // cos(2 pi q / 64), any q >= 0
     const int m = q & 63;
     return m <= 16 ? cos64(m) : m <= 32 ? -cos64(32 - m) : m <= 48 ? -cos64(m - 32) : cos64(64 - m);
 }
-__host__ __device__ constexpr float sin_turn64(int q) { return cos_turn64(q + 48); }
+__host__ __device__ constexpr double sin_turn64(int q) { return cos_turn64(q + 48); }
 
 // b * exp(-+2 pi i m / 64) (INV: +), m a constant after unrolling
 template <bool INV>
@@ -81,14 +82,14 @@ __device__ __forceinline__ float2 rot64(float2 b, int m) {
     if (m == 16) return INV ? make_float2(-b.y, b.x) : make_float2(b.y, -b.x);
     if (m == 32) return make_float2(-b.x, -b.y);
     if (m == 48) return INV ? make_float2(b.y, -b.x) : make_float2(-b.y, b.x);
-    constexpr float h = cos64(8);
+    constexpr float h = (float)cos64(8);
     if (m == 8)
         return INV ? make_float2((b.x - b.y) * h, (b.x + b.y) * h)
                    : make_float2((b.x + b.y) * h, (b.y - b.x) * h);
     if (m == 24)
         return INV ? make_float2((b.x + b.y) * -h, (b.x - b.y) * h)
                    : make_float2((b.y - b.x) * h, (b.x + b.y) * -h);
-    const float c = cos_turn64(m), s = INV ? sin_turn64(m) : -sin_turn64(m);
+    const float c = (float)cos_turn64(m), s = (float)(INV ? sin_turn64(m) : -sin_turn64(m));
     return make_float2(fmaf(b.x, c, -b.y * s), fmaf(b.x, s, b.y * c));
 }
 
@@ -108,6 +109,36 @@ __host__ __device__ constexpr int brev(int i) {
     return o;
 }
 
+// lo, hi = lo + w hi, lo - w hi, w = exp(-+2 pi i m / 64), 0 <= m < 32.  A
+// rotation that is no quarter turn takes two FMAs for (x + r y, y - r x) with
+// the ratio r of its sine and cosine (at most 1) and four for the sums scaled
+// by the larger of the two: six operations and two roundings per result,
+// against eight and three for the product and its sum and difference.
+template <bool INV>
+__device__ __forceinline__ void butterfly(float2 &lo, float2 &hi, int m) {
+    const float2 a = lo, b = hi;
+    if (m % 16 == 0) {
+        const float2 t = rot64<INV>(b, m);
+        hi = csub(a, t);
+        lo = cadd(a, t);
+        return;
+    }
+    const double c = cos_turn64(m), s = INV ? -sin_turn64(m) : sin_turn64(m);
+    float2 t;
+    float k;
+    if (m <= 8 || m >= 24) {
+        const float r = (float)(s / c);
+        t = make_float2(fmaf(r, b.y, b.x), fmaf(-r, b.x, b.y));
+        k = (float)c;
+    } else {
+        const float r = (float)(c / s);
+        t = make_float2(fmaf(r, b.x, b.y), fmaf(r, b.y, -b.x));
+        k = (float)s;
+    }
+    hi = make_float2(fmaf(-k, t.x, a.x), fmaf(-k, t.y, a.y));
+    lo = make_float2(fmaf(k, t.x, a.x), fmaf(k, t.y, a.y));
+}
+
 // R-point DFT (sign -, or + with INV; unnormalised) of v[0..R), in place:
 // input in natural order, bin r of the result in v[brev<R>(r)].  Radix-2
 // decimation in time over the bit-reversed view, so nothing is moved.
@@ -119,10 +150,7 @@ __device__ __forceinline__ void dft(float2 *v) {
         for (int i = 0; i < R; i += 2 * h) {
 #pragma unroll
             for (int q = 0; q < h; ++q) {
-                float2 &lo = v[brev<R>(i + q)], &hi = v[brev<R>(i + q + h)];
-                const float2 b = rot64<INV>(hi, q * (32 / h));
-                hi = csub(lo, b);
-                lo = cadd(lo, b);
+                butterfly<INV>(v[brev<R>(i + q)], v[brev<R>(i + q + h)], q * (32 / h));
             }
         }
     }
@@ -138,7 +166,18 @@ struct Plan {
     static constexpr int BUF = M + M / EPT;      // padded points of the buffer
     static constexpr int TW1 = (RA - 1) * T, TW2 = (RB - 1) * RC;     // table entries
     static_assert(RA * RB * RC == M && EPT % RA == 0 && EPT % RB == 0 && EPT % RC == 0, "digits");
-    static __device__ __forceinline__ int pad(int i) { return i + i / EPT; }
+    static __host__ __device__ __forceinline__ constexpr int pad(int i) { return i + i / EPT; }
+    // pad(j + k) for a constant k; pj = pad(j).  Where EPT divides k the two
+    // add up, and an access is a register plus an immediate.
+    static __device__ __forceinline__ int pad_from(int pj, int j, int k) {
+        return k % EPT == 0 ? pj + pad(k) : pad(j + k);
+    }
+    // pad(c / RC * RB RC + c mod RC + r RC), element r of DFT c of pass 2:
+    // base(c) + step(r) where EPT divides RB RC
+    static __device__ __forceinline__ int pass2(int c, int r) {
+        if (RB * RC % EPT == 0) return c / RC * pad(RB * RC) + c % RC + pad(r * RC);
+        return pad(c / RC * (RB * RC) + c % RC + r * RC);
+    }
 };
 
 // Tables of a plan: tw1[(r - 1) T + d] = exp(-2 pi i r (d + shift) / M), d < T,
@@ -169,10 +208,11 @@ struct Tw1 {
     }
 };
 
-// The point held in v[i] by thread j of a line, before and after conv().
+// Thread j of a line holds point j + point_of(i) in v[i], before and after
+// conv().
 template <class P>
-__device__ __forceinline__ int point_of(int j, int i) {
-    return j + (i / P::RA) * P::T + (i % P::RA) * P::CA;
+__device__ __forceinline__ constexpr int point_of(int i) {
+    return (i / P::RA) * P::T + (i % P::RA) * P::CA;
 }
 
 // Barrier of the threads of one line; `slot` tells the lines of a CTA apart.
@@ -203,7 +243,7 @@ template <class P>
 struct Filter {
     const float2 *h;
     __device__ __forceinline__ float2 operator()(float2 z, int i, int j) const {
-        return cmul(z, __ldg(h + i * P::T + j));
+        return cmul(z, h[i * P::T + j]);
     }
 };
 // Bin held as element i of thread j in the middle pass.
@@ -214,7 +254,7 @@ inline int spectrum_order(int i, int j) {
     return k0 + P::RA * (k1 + P::RB * k2);
 }
 
-// v: points point_of(j, i), replaced by the convolved line's at the same
+// v: points j + point_of(i), replaced by the convolved line's at the same
 // places.  buf: P::BUF points of this line's own.  tw1(r, j, g)
 // (column d = j + g T), tw2: forward twiddles; iw1, iw2: those of the inverse (conjugated here).  The caller's next use of
 // `buf` (by this function too) must be behind a line_sync.
@@ -222,29 +262,29 @@ template <class P, class Tw, class Mul>
 __device__ __forceinline__ void conv(float2 (&v)[P::EPT], float2 *buf, int j, int slot, bool alone,
                                      const Tw &tw1, const float2 *tw2, const Tw &iw1,
                                      const float2 *iw2, const Mul &mul) {
+    const int pj = P::pad(j);
     // pass 1, from registers
 #pragma unroll
     for (int g = 0; g < P::GA; ++g) {
-        const int d = j + g * P::T;
         dft<P::RA, false>(v + g * P::RA);
 #pragma unroll
         for (int r = 0; r < P::RA; ++r) {
             const float2 z = v[g * P::RA + brev<P::RA>(r)];
-            buf[P::pad(d + r * P::CA)] = r ? cmul(z, tw1(r, j, g)) : z;
+            buf[P::pad_from(pj, j, g * P::T + r * P::CA)] = r ? cmul(z, tw1(r, j, g)) : z;
         }
     }
     line_sync<P>(slot, alone);
     // pass 2: DFT c covers points k0 RB RC + n1 RC + n2, k0 = c / RC, n2 = c mod RC
 #pragma unroll
     for (int g = 0; g < P::GB; ++g) {
-        const int c = j + g * P::T, n2 = c % P::RC, at = (c / P::RC) * (P::RB * P::RC) + n2;
+        const int c = j + g * P::T, n2 = c % P::RC;
 #pragma unroll
-        for (int r = 0; r < P::RB; ++r) v[r] = buf[P::pad(at + r * P::RC)];
+        for (int r = 0; r < P::RB; ++r) v[r] = buf[P::pass2(c, r)];
         dft<P::RB, false>(v);
 #pragma unroll
         for (int r = 0; r < P::RB; ++r) {
             const float2 z = v[brev<P::RB>(r)];
-            buf[P::pad(at + r * P::RC)] = r ? cmul(z, tw2[(r - 1) * P::RC + n2]) : z;
+            buf[P::pass2(c, r)] = r ? cmul(z, tw2[(r - 1) * P::RC + n2]) : z;
         }
     }
     line_sync<P>(slot, alone);
@@ -269,25 +309,24 @@ __device__ __forceinline__ void conv(float2 (&v)[P::EPT], float2 *buf, int j, in
     // inverse of pass 2
 #pragma unroll
     for (int g = 0; g < P::GB; ++g) {
-        const int c = j + g * P::T, n2 = c % P::RC, at = (c / P::RC) * (P::RB * P::RC) + n2;
+        const int c = j + g * P::T, n2 = c % P::RC;
 #pragma unroll
         for (int r = 0; r < P::RB; ++r) {
-            const float2 z = buf[P::pad(at + r * P::RC)];
+            const float2 z = buf[P::pass2(c, r)];
             v[r] = r ? cmulc(z, iw2[(r - 1) * P::RC + n2]) : z;
         }
         dft<P::RB, true>(v);
 #pragma unroll
-        for (int r = 0; r < P::RB; ++r) buf[P::pad(at + r * P::RC)] = v[brev<P::RB>(r)];
+        for (int r = 0; r < P::RB; ++r) buf[P::pass2(c, r)] = v[brev<P::RB>(r)];
     }
     line_sync<P>(slot, alone);
     // inverse of pass 1, into registers in natural order
 #pragma unroll
     for (int g = 0; g < P::GA; ++g) {
-        const int d = j + g * P::T;
         float2 u[P::RA];
 #pragma unroll
         for (int r = 0; r < P::RA; ++r) {
-            const float2 z = buf[P::pad(d + r * P::CA)];
+            const float2 z = buf[P::pad_from(pj, j, g * P::T + r * P::CA)];
             u[r] = r ? cmulc(z, iw1(r, j, g)) : z;
         }
         dft<P::RA, true>(u);

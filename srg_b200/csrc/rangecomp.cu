@@ -10,7 +10,7 @@
 // go through in blocks: one kernel pads a block, cuFFT transforms it, one
 // kernel multiplies, cuFFT transforms back, one kernel writes the valid
 // samples.  FFTs by cuFFT (the reference uses FFTW in single precision).
-// Pulses of up to 4,096 samples (Sentinel-1 IW: ~3,370) take the fused
+// Pulses of up to about 6,800 samples (Sentinel-1 IW: ~3,370) take the fused
 // overlap-save kernel instead (rc_os_kernel below), same samples.
 #include <cuda_runtime.h>
 #include <cufft.h>
@@ -23,8 +23,8 @@
 #include <vector>
 
 #include "../../include/srg_bp.h"
+#include "fft_conv.cuh"
 #include "host_internal.h"
-#include "smem_fft.cuh"
 
 using namespace srg;
 using namespace srg::detail;
@@ -85,89 +85,67 @@ __global__ void rc_out_kernel(const float2 *__restrict__ buf, int l0, int nlines
 // linear correlation (the 32,768-point circular one never wraps into them),
 // so 8,192-point transforms give them exactly up to rounding: a segment of
 // 8,192 samples from s0 (zeros past the line) yields y[s0 .. s0 + L),
-// L = 8192 - npts + 1.  A CTA (one per SM, persistent) takes (line,
-// segment) items in turn: it loads the segment's samples once, transforms
-// them in shared memory, multiplies by the filter
-// H = (32768 / 8192) conj(DFT_8192(r)), transforms back (a forward transform
-// of the conjugate, conjugated) and writes its L outputs once: the lines
-// cross HBM once each way, where the cuFFT path below takes five passes over
-// 32,768-point rows.  Transforms: Stockham autosort passes of radix 16, 16,
-// 16 and 2 (16 values per thread per pass), each DFT in registers, the
-// padded shared layout i + i / 16 keeping the 16-strided accesses off common
-// banks, the twiddles of each pass from its own table in shared memory
-// (exactly rounded, laid out so that a warp reads consecutive entries),
-// loaded once per CTA.  Pulses of more than 4,096 samples take the cuFFT
-// path.
-constexpr int kOsM = 8192;                       // segment transform
-constexpr int kOsMaxPts = kOsM / 2;              // longest pulse the segments take
-constexpr int kOsBuf = smem_fft::kBuf;          // padded segment (float2)
-constexpr int kOsThreads = smem_fft::kThreads;   // one radix-16 work item per thread
-constexpr int kOsTw16 = smem_fft::kTw16, kOsTw256 = smem_fft::kTw256, kOsTw2 = smem_fft::kTw2;
-constexpr int kOsTw = smem_fft::kTw;
-constexpr int kOsSmem = (kOsBuf + kOsTw) * (int)sizeof(float2);
-using smem_fft::brev;
-using smem_fft::cadd;
-using smem_fft::cconj;
-using smem_fft::cmul;
-using smem_fft::csub;
-using smem_fft::dft;
-__device__ __forceinline__ int os_pad(int i) { return smem_fft::pad(i); }
-__device__ __forceinline__ void os_pass(float2 *buf, int Ns, const float2 *tw) {
-    smem_fft::pass16<kOsM>(buf, Ns, tw);
-}
+// L = 8192 - npts + 1.  A CTA (one per SM, persistent) takes (line, segment)
+// items in turn: it loads the segment's samples once, convolves them in shared
+// memory (fft_conv.cuh) with the filter H = (32768 / 8192) conj(DFT_8192(r))
+// and writes its L outputs once: the lines cross HBM once each way, where the
+// cuFFT path below takes five passes over 32,768-point rows.  A CTA takes two
+// segments at once, 256 threads each, that share the filter's spectrum (64 KB)
+// and pass 1's twiddles (30 KB) in shared memory.  Bound by instruction issue
+// (see fft_conv.cuh): 1,500 lines of 24,000 samples, pulse of 3,371, take
+// 0.30 ms (0.45 with self-sorting transforms of one segment per 512-thread CTA),
+// 700 lines of 29,001 with a pulse of 5,147 0.23 ms (0.58 with cuFFT).  The same
+// with the tables read through L1 and two CTAs per SM: 0.31 ms; as two halves
+// of 4,096 points at 16 points per thread: 0.42 ms.
+using Seg = fftc::Plan<8192, 32, 16, 16, 32>;
+constexpr int kOsM = Seg::M;                     // segment transform
+// Segments per line up to which the kernel is the faster path: one takes
+// 41 ns (of the whole chip), a line of the cuFFT path 0.84 us whatever its
+// pulse.  Pulses of up to 6,400 samples stay within it on lines of any length.
+constexpr int kOsMaxSegs = 20;
+constexpr int kOsLines = 2;                      // segments of a CTA at once
+constexpr int kOsThreads = kOsLines * Seg::T;
+constexpr int kOsSmem = (kOsLines * Seg::BUF + kOsM + Seg::TW1) * (int)sizeof(float2);
 
-// Persistent: each CTA takes segments (line, s0) in turn, after loading the
-// twiddle tables once.
 __global__ void __launch_bounds__(kOsThreads, 1)
 rc_os_kernel(const float2 *__restrict__ in, long long ld_in, int nsamps, int nvalid, int L,
-             int nseg, int nitems, const float2 *__restrict__ H, const float2 *__restrict__ twg,
+             int nseg, int nitems, const float2 *__restrict__ H, const float2 *__restrict__ tw,
              float2 *__restrict__ out, long long ld_out) {
     extern __shared__ float2 os_sm[];
-    float2 *buf = os_sm, *tw = os_sm + kOsBuf;
-    const int t = threadIdx.x;
-    for (int i = t; i < kOsTw; i += kOsThreads) tw[i] = __ldg(twg + i);
-    for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+    const int j = threadIdx.x % Seg::T, slot = threadIdx.x / Seg::T;
+    float2 *buf = os_sm + slot * Seg::BUF;
+    float2 *h = os_sm + kOsLines * Seg::BUF, *t1 = h + kOsM;
+    for (int i = threadIdx.x; i < kOsM; i += kOsThreads) h[i] = __ldg(H + i);
+    for (int i = threadIdx.x; i < Seg::TW1; i += kOsThreads) t1[i] = __ldg(tw + i);
+    __syncthreads();
+    const fftc::Tw1<Seg> tw1{t1};
+    const fftc::Filter<Seg> filter{h};
+    const int step = gridDim.x * kOsLines;
+    for (int item = blockIdx.x * kOsLines + slot; item < nitems; item += step) {
         const int line = item / nseg, s0 = (item - line * nseg) * L;
-        const float2 *x = in + (long long)line * ld_in;
-        // forward transform, pass 1 (Ns = 1) straight from the line
-        {
-            float2 v[16];
+        const float2 *x = in + (long long)line * ld_in + s0 + j;
+        const int nin = nsamps - s0 - j;
+        float2 v[Seg::EPT];
 #pragma unroll
-            for (int r = 0; r < 16; ++r) {
-                const int i = s0 + t + r * kOsThreads;
-                v[r] = i < nsamps ? __ldg(x + i) : make_float2(0.f, 0.f);
-            }
-            dft<16>(v);
-#pragma unroll
-            for (int r = 0; r < 16; ++r) buf[os_pad(t * 16 + r)] = v[brev<16>(r)];
+        for (int i = 0; i < Seg::EPT; ++i) {
+            const int n = fftc::point_of<Seg>(i);
+            v[i] = n < nin ? fftc::ld_stream(x + n) : make_float2(0.f, 0.f);
         }
-        __syncthreads();  // (the first time also the tables)
-        os_pass(buf, 16, tw + kOsTw16);
-        os_pass(buf, 256, tw + kOsTw256);
-        // last pass (radix 2, Ns = 4096): each item touches only its own pair,
-        // so the filter and the conjugation of the inverse go in place
-#pragma unroll
-        for (int it = 0; it < kOsM / 2 / kOsThreads; ++it) {
-            const int j = t + it * kOsThreads;
-            const float2 a = buf[os_pad(j)], b = cmul(buf[os_pad(j + kOsM / 2)], tw[kOsTw2 + j]);
-            buf[os_pad(j)] = cconj(cmul(cadd(a, b), __ldg(H + j)));
-            buf[os_pad(j + kOsM / 2)] = cconj(cmul(csub(a, b), __ldg(H + j + kOsM / 2)));
+        if (item + step < nitems) {  // the next segment into L2
+            const int nl = (item + step) / nseg, ns = (item + step - nl * nseg) * L;
+            const float2 *nx = in + (long long)nl * ld_in + ns;
+            for (int c = 16 * j; c < min(kOsM, nsamps - ns); c += 16 * Seg::T)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + c));
         }
-        __syncthreads();
-        // inverse: forward transform of the conjugate
-        os_pass(buf, 1, nullptr);
-        os_pass(buf, 16, tw + kOsTw16);
-        os_pass(buf, 256, tw + kOsTw256);
-        float2 *y = out + (long long)line * ld_out + s0;
-        const int nout = min(L, nvalid - s0);
+        fftc::conv<Seg>(v, buf, j, slot, false, tw1, tw + Seg::TW1, tw1, tw + Seg::TW1, filter);
+        float2 *y = out + (long long)line * ld_out + s0 + j;
+        const int nout = min(L, nvalid - s0) - j;
 #pragma unroll
-        for (int it = 0; it < kOsM / 2 / kOsThreads; ++it) {
-            const int j = t + it * kOsThreads;
-            const float2 a = buf[os_pad(j)], b = cmul(buf[os_pad(j + kOsM / 2)], tw[kOsTw2 + j]);
-            if (j < nout) y[j] = cconj(cadd(a, b));
-            if (j + kOsM / 2 < nout) y[j + kOsM / 2] = cconj(csub(a, b));
+        for (int i = 0; i < Seg::EPT; ++i) {
+            const int n = fftc::point_of<Seg>(i);
+            if (n < nout) y[n] = v[i];
         }
-        __syncthreads();  // the segment's reads are done before the next one's writes
+        fftc::line_sync<Seg>(slot, false);  // the buffer's reads are done
     }
 }
 
@@ -203,7 +181,7 @@ struct RcCtx {
     // overlap-save path: filter spectrum, twiddle tables, their parameters
     DevBuf os_h, os_tw;
     bool os_ready = false;
-    int sms = 0;
+    int os_ctas = 0;  // resident CTAs
     float os_key[4] = {NAN, NAN, NAN, NAN};
 };
 RcCtx g_rc[64];
@@ -252,16 +230,21 @@ int srg_range_compress_device(const float *lines, long long ld_in, int nlines, i
     RcCtx &x = g_rc[dev];
     std::lock_guard<std::mutex> g(x.mu);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (npts <= kOsMaxPts) {
+    const int L = kOsM - npts + 1, nseg = L > 0 ? (nvalid + L - 1) / L : 0;
+    if (nseg > 0 && nseg <= kOsMaxSegs) {
         // fused overlap-save kernel (see rc_os_kernel)
-        if ((rc = x.os_h.ensure(sizeof(float2) * kOsM)) || (rc = x.os_tw.ensure(sizeof(float2) * kOsTw)))
+        if ((rc = x.os_h.ensure(sizeof(float2) * kOsM)) ||
+            (rc = x.os_tw.ensure(sizeof(float2) * (Seg::TW1 + Seg::TW2))))
             return rc;
-        const double pi = 4.0 * std::atan2(1.0, 1.0);
         if (!x.os_ready) {
-            const std::vector<float2> tw = smem_fft::twiddle_tables();
+            const std::vector<float2> tw = fftc::tables<Seg>(0.0);
+            int sms = 0;
             CKR(cudaFuncSetAttribute(rc_os_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kOsSmem));
-            CKR(cudaDeviceGetAttribute(&x.sms, cudaDevAttrMultiProcessorCount, dev));
-            CKR(cudaMemcpyAsync(x.os_tw.p, tw.data(), sizeof(float2) * kOsTw, cudaMemcpyHostToDevice, st));
+            CKR(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+            CKR(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&x.os_ctas, rc_os_kernel, kOsThreads, kOsSmem));
+            if (x.os_ctas < 1) return fail(SRG_E_UNSUPPORTED, "segment transform does not fit an SM");
+            x.os_ctas *= sms;
+            CKR(cudaMemcpyAsync(x.os_tw.p, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice, st));
             CKR(cudaStreamSynchronize(st));  // `tw` is pageable host memory that goes out of scope
             x.os_ready = true;
         }
@@ -274,17 +257,18 @@ int srg_range_compress_device(const float *lines, long long ld_in, int nlines, i
             host_fft(a);
             std::vector<float2> h(kOsM);
             const double scale = (double)kRangeFFT / kOsM;
-            for (int k = 0; k < kOsM; ++k)
-                h[k] = make_float2((float)(scale * a[k].real()), (float)(-scale * a[k].imag()));
+            for (int i = 0; i < Seg::EPT; ++i)
+                for (int j = 0; j < Seg::T; ++j) {
+                    const std::complex<double> b = a[fftc::spectrum_order<Seg>(i, j)];
+                    h[i * Seg::T + j] = make_float2((float)(scale * b.real()), (float)(-scale * b.imag()));
+                }
             CKR(cudaMemcpyAsync(x.os_h.p, h.data(), sizeof(float2) * kOsM, cudaMemcpyHostToDevice, st));
             CKR(cudaStreamSynchronize(st));  // `h` is pageable host memory that goes out of scope
             std::memcpy(x.os_key, key, sizeof key);
         }
-        const int L = kOsM - npts + 1;
-        const int nseg = (nvalid + L - 1) / L;
         if ((long long)nlines * nseg > INT_MAX) return fail(SRG_E_ARG, "too many lines: %d", nlines);
         const int nitems = nlines * nseg;
-        rc_os_kernel<<<std::min(nitems, x.sms), kOsThreads, kOsSmem, st>>>(
+        rc_os_kernel<<<std::min((nitems + kOsLines - 1) / kOsLines, x.os_ctas), kOsThreads, kOsSmem, st>>>(
             reinterpret_cast<const float2 *>(lines), ld_in, nsamps, nvalid, L, nseg, nitems,
             static_cast<const float2 *>(x.os_h.p), static_cast<const float2 *>(x.os_tw.p),
             reinterpret_cast<float2 *>(out), ld_out);
