@@ -37,7 +37,10 @@ extern "C" {
 
 typedef struct srg_bp_options {
     int form;          /* SRG_FORM_FP64 or SRG_FORM_SPLIT */
-    int tile_cfg;      /* kernel shape index (srg_tile_config_count()); -1: tuned default */
+    int tile_cfg;      /* kernel shape index (srg_tile_config_count()); -1: the
+                          default for the form and the bursts (coarse grids,
+                          oversampled lines and odd row strides take a twin of
+                          the first shape with the same results) */
     int device;        /* CUDA device ordinal; -1: current device */
     int centres_on_host; /* must be 0: the per-line azimuth centres are solved
                             on the GPU (1 is SRG_E_UNSUPPORTED wherever the

@@ -70,6 +70,7 @@ struct __align__(16) StageHdr {
     float p0, p1, p2;     // as phase (rad), p0 in [-pi, pi]
     float u0x, u0y, u0z;  // u_{j+1} - u_j = u0 + j us (j = pulse index within the chunk)
     float usx, usy, usz;
+    int split;     // WIDE: 0, or the chunk fills wide windows (2: no tap leaves them)
 };
 
 struct CtlWS {
@@ -150,6 +151,15 @@ __device__ __forceinline__ unsigned tap_index(float tm) {
     else return min(__float_as_uint(tm) - (unsigned)kFloorMagicBits, (unsigned)(WB - 2));
 }
 
+// *p where `use`, else `v`, without a branch.
+__device__ __forceinline__ float2 ld_where(bool use, const float2 *p, float2 v) {
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\t"
+        "@q ld.global.nc.v2.f32 {%0, %1}, [%3];\n\t}"
+        : "+f"(v.x), "+f"(v.y)
+        : "r"((int)use), "l"(p));
+    return v;
+}
+
 // Chunk schedule of a tile: the pulse range [kmin, kmax) is cut at ka and kb
 // (the interior segment [ka, kb) lies inside every formed pixel's aperture)
 // and each of the three segments into chunks of at most CK pulses, so that
@@ -191,7 +201,19 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
 // GATE: the range lines may still be uploading (BurstDev::ready); the
 // producer waits for each chunk's rows.  A separate instantiation, because
 // the wait's code alone costs the ungated kernel ~4 % (measured).
-template <int FORM, int TX, int TY, int NC, int CK, int NS, int WB, int MINB, bool GATE = false>
+// WIDE (split form): a chunk whose pixels spread over more bins than the window
+// (coarse grids, oversampled lines, steep relief) but at most kWideBins goes
+// through two stages of kWideRows pulses by kWideBins bins instead of one, by a
+// second TMA descriptor (tmaps[nbursts + burst]); beyond that the taps outside
+// the window are read from global memory by predicated loads, four pulses at
+// a time.  Same terms, order and rounding as the kernel without it, where
+// every such tap waits for a load of its own under a branch: a burst of 1,500
+// pulses on lines oversampled 2x takes 0.99 against 2.82 ms, a 256 x 256 grid at
+// 2e-4 deg (few tiles, latency alone) 0.27 against 0.69.  It also stages lines
+// without a TMA descriptor by asynchronous copies.  A separate instantiation:
+// that code alone costs the default shape 1.7 %.
+template <int FORM, int TX, int TY, int NC, int CK, int NS, int WB, int MINB, bool GATE = false,
+          bool WIDE = false>
 __global__ void __launch_bounds__((NC + 1) * 32, MINB)
 bp_ws(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
       const CUtensorMap *__restrict__ tmaps, int *__restrict__ work_counter,
@@ -474,6 +496,7 @@ bp_ws(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
         const int nchunks = plan.count();
         const bool use_tma = B.tmap >= 0;
 
+        uint32_t extra = 0;  // second stages of wide chunks so far in this tile
         issued = 0;
         if (producer) {
             // ---- producer warp ----
@@ -508,9 +531,9 @@ bp_ws(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
                 nsz = sp[2];
             }
             for (int c = 0; c < nchunks; ++c) {
-                const uint32_t g = gchunk + c;
-                const int s = g % NS;
-                const uint32_t r = g / NS;
+                uint32_t g = gchunk + c + extra;
+                int s = g % NS;
+                uint32_t r = g / NS;
                 int k0, nk;
                 plan.chunk(c, CK, k0, nk);
                 const int k = min(k0 + lane, Pm1);
@@ -554,6 +577,10 @@ bp_ws(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
                     const bool bounded = __int_as_float(devmax) < 0.5f;
                     hv.fast = (rangeok && bounded && need <= WB) ? 1 : 0;
                     hv.interior = interior ? 1 : 0;
+                    if constexpr (WIDE) {
+                        const bool wideok = x0 >= 1 && (double)(x0 + kWideBins) <= rmaxb - 1.0;
+                        hv.split = need > WB && need <= kWideBins ? (wideok && bounded ? 2 : 1) : 0;
+                    }
                 }
                 hv.tlo = (float)(-(double)x0);
                 hv.thi = __double2float_rn(rmaxb - (double)x0);
@@ -635,8 +662,20 @@ bp_ws(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
                         __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(act ? err : 0.f)));
                     hv.poly = (nk >= 3 && (double)resmax * kTwoPi * Kc < kPolyTolRad) ? 1 : 0;
                 }
+                // one stage, or two for a wide chunk
+                const int parts = WIDE && hv.split && nk > kWideRows ? 2 : 1;
+                bool gave_up = false;
+#pragma unroll 1
+                for (int part = 0; part < parts; ++part) {
+                if (WIDE && part) {
+                    ++extra;
+                    ++g;
+                    s = g % NS;
+                    r = g / NS;
+                }
                 if (!mbar_wait_bounded(&ctl.empty[s], (r & 1) ^ 1, ctl.spin)) {
                     ctl.abort = 1;
+                    gave_up = true;
                     break;
                 }
                 // Range lines still in transfer: wait (bounded) until the rows
@@ -647,6 +686,7 @@ bp_ws(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
                         if (!wait_word_at_least(ready, target, ctl.spin)) {
                             if (lane == 0) atomicOr(err, ERR_UPLOAD_TIMEOUT);
                             ctl.abort = 1;
+                            gave_up = true;
                             break;
                         }
                         // the rows were seen through a generic-proxy acquire;
@@ -660,11 +700,20 @@ bp_ws(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
                 // without arriving; the phase still needs all 32 lane arrivals
                 // below, which follow those writes.
                 if (lane == 0 && use_tma) {
-                    if (c == 0) fence_tensormap_acquire(tmaps + tmap_i);
+                    if (c == 0) {
+                        fence_tensormap_acquire(tmaps + tmap_i);
+                        if (WIDE) fence_tensormap_acquire(tmaps + nbursts + tmap_i);
+                    }
                     fence_proxy_async_shared();
-                    mbar_expect_tx(&ctl.full[s], (uint32_t)(WB * CK * 8));
-                    tma_load_2d(samp0 + (size_t)s * CK * WB, tmaps + tmap_i, &ctl.full[s],
-                                x0 - bin0, k0);
+                    if (WIDE && hv.split) {
+                        mbar_expect_tx(&ctl.full[s], (uint32_t)(kWideBins * kWideRows * 8));
+                        tma_load_2d(samp0 + (size_t)s * CK * WB, tmaps + nbursts + tmap_i, &ctl.full[s],
+                                    x0 - bin0, k0 + part * kWideRows);
+                    } else {
+                        mbar_expect_tx(&ctl.full[s], (uint32_t)(WB * CK * 8));
+                        tma_load_2d(samp0 + (size_t)s * CK * WB, tmaps + tmap_i, &ctl.full[s],
+                                    x0 - bin0, k0);
+                    }
                     issued |= 1u << s;
                     issued_par = (issued_par & ~(1u << s)) | ((r & 1u) << s);
                 }
@@ -677,23 +726,34 @@ bp_ws(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
                     }
                 }
                 if constexpr (FORM == FORM_SPLIT) {
-                    if (lane < CK) {
-                        PP &p = prm[s * CK + lane];
+                    const int at = WIDE ? lane - part * kWideRows : lane;
+                    if (lane < CK && at >= 0) {
+                        PP &p = prm[s * CK + at];
                         p.a = pa;
                         p.b = make_float4(pb, 0.f, 0.f, 0.f);
                     }
                 }
                 if (lane == 0) hdr[s] = hv;
                 if (!use_tma) {
-                    // no TMA descriptor for this burst: stage the window with plain loads
+                    // no TMA descriptor for this burst
                     float2 *w = samp0 + (size_t)s * CK * WB;
-                    for (int idx = lane; idx < CK * WB; idx += 32) {
-                        const int j = idx / WB;
-                        w[idx] = ld_sample(B, k0 + j, x0 + (idx - j * WB));
+                    if constexpr (WIDE) {
+                        // single asynchronous copies, which the stage's phase
+                        // also waits for
+                        stage_samples(B, w, k0 + part * kWideRows, hv.split ? kWideRows : CK, x0,
+                                      hv.split ? kWideBins : WB, lane, 32);
+                        cp_async_arrive(&ctl.full[s]);
+                    } else {
+                        for (int idx = lane; idx < CK * WB; idx += 32) {
+                            const int j = idx / WB;
+                            w[idx] = ld_sample(B, k0 + j, x0 + (idx - j * WB));
+                        }
                     }
                 }
                 __syncwarp();
                 mbar_arrive(&ctl.full[s]);
+                }
+                if (gave_up) break;
             }
             if (lane == 0) ctl.item = atomicAdd(work_counter, 1);
         } else {
@@ -702,8 +762,8 @@ bp_ws(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
             const float invd_c = B.inv_dmrg_f, Kr_c = (float)(kTwoPi * B.K);
             const double rng0_c = B.rngstart, rmax_c = B.rmax, dmrg_c = B.dmrg, k4pi_c = B.k4pi;
             for (int c = 0; c < nchunks; ++c) {
-                const uint32_t g = gchunk + c;
-                const int s = g % NS;
+                uint32_t g = gchunk + c + extra;
+                int s = g % NS;
                 const uint32_t r = g / NS;
                 if (!mbar_wait_bounded(&ctl.full[s], r & 1, ctl.spin)) {
                     ctl.abort = 1;
@@ -849,7 +909,84 @@ bp_ws(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
                         uacc[m] = dwa[m] + dr0[m];
                         cphp[m] = fmaf(dr0[m], Kr, cph[m]);
                     }
-                    if (h.fast && h.interior) {
+                    if (WIDE && !h.fast) {
+                        // Chunks with taps outside the window: two wide stages,
+                        // or the window and global memory.  No branch in the
+                        // loop, so four pulses' taps are in flight.
+                        const float2 *line = B.burst + ((long long)k0 * B.ldb - B.bin0);
+                        const long long ldb = B.ldb;
+                        const int lo = B.bin0, hi = min(B.bin0 + B.nbins, B.S);
+                        auto pulses = [&](auto proven, int j0, int j1) {
+                            constexpr bool PROVEN = decltype(proven)::value;
+                            const int wb = h.split ? kWideBins : WB;
+#pragma unroll 4
+                            for (int j = j0; j < j1; ++j) {
+                                const int k = k0 + j;
+                                const float4 pa = pp[j - j0].a;
+                                const float rb = pp[j - j0].b.x;
+                                const float2 *row = win + (j - j0) * wb;
+#pragma unroll
+                                for (int m = 0; m < M; ++m) {
+                                    const float dwp = fmaf(d[m][0], pa.x, fmaf(d[m][1], pa.y, fmaf(d[m][2], pa.z, gsl[m])));
+                                    const float t = fmaf(whi[m] + uacc[m], invd, rb);
+                                    const float ph = cphp[m] + pa.w;
+                                    uacc[m] += dwp;
+                                    cphp[m] = fmaf(dwp, Kr, cphp[m]);
+                                    const float fl = floorf(t);
+                                    const int i = (int)fl;
+                                    const float fr = t - fl;
+                                    bool ok = (k >= azs[m]) & (k < aze[m]);
+                                    float2 s0, s1;
+                                    if constexpr (PROVEN) {  // bounded for memory safety
+                                        const int ic = min(max(i, 0), kWideBins - 2);
+                                        s0 = row[ic];
+                                        s1 = row[ic + 1];
+                                    } else {
+                                        ok = ok & (t >= h.tlo) & (t <= h.thi);
+                                        const bool in = (unsigned)i < (unsigned)(wb - 1);
+                                        const int is = in ? i : 0, gi = i + h.x0;
+                                        const float2 zero = make_float2(0.f, 0.f);
+                                        s0 = in ? row[is] : zero;
+                                        s1 = in ? row[is + 1] : zero;
+                                        const float2 *q = line + ((long long)j * ldb + gi);
+                                        s0 = ld_where(ok & !in & (gi >= lo) & (gi < hi), q, s0);
+                                        s1 = ld_where(ok & !in & (gi + 1 >= lo) & (gi + 1 < hi), q + 1, s1);
+                                    }
+                                    float vr = fmaf(fr, s1.x - s0.x, s0.x);
+                                    float vi = fmaf(fr, s1.y - s0.y, s0.y);
+                                    vr = ok ? vr : 0.f;
+                                    vi = ok ? vi : 0.f;
+                                    float sn, cs;
+                                    __sincosf(ph, &sn, &cs);
+                                    accr[m] = fmaf(vr, cs, fmaf(-vi, sn, accr[m]));
+                                    acci[m] = fmaf(vr, sn, fmaf(vi, cs, acci[m]));
+                                }
+                            }
+                        };
+                        bool gave_up = false;
+#pragma unroll 1
+                        for (int j0 = 0;; j0 += kWideRows) {
+                            const int j1 = h.split ? min(nk, j0 + kWideRows) : nk;
+                            if (h.split == 2) pulses(std::true_type{}, j0, j1);
+                            else pulses(std::false_type{}, j0, j1);
+                            if (j1 == nk) break;
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(&ctl.empty[s]);
+                            ++extra;
+                            ++g;
+                            s = g % NS;
+                            if (!mbar_wait_bounded(&ctl.full[s], (g / NS) & 1, ctl.spin)) {
+                                gave_up = true;
+                                break;
+                            }
+                            win = samp0 + (size_t)s * CK * WB;
+                            pp = prm + s * CK;
+                        }
+                        if (gave_up) {
+                            ctl.abort = 1;
+                            break;
+                        }
+                    } else if (h.fast && h.interior) {
                         // consecutive pulses share only the two accumulators, so
                         // unrolling gives the scheduler independent terms
 #pragma unroll 2
@@ -998,12 +1135,13 @@ bp_ws(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
                 if (GATE && B.rb_done) __threadfence();
             }
         }
-        gchunk += nchunks;
+        gchunk += nchunks + extra;
         __syncthreads();
         if (ctl.abort) {
             if (tid == 0) atomicOr(err, ERR_TMA_TIMEOUT);
             // let the copies this CTA issued drain before it leaves (bounded by
             // the default limit whatever the launch's: a copy in flight ends in us)
+            if (WIDE && producer) cp_async_wait_all();
             if (producer && lane == 0) {
                 for (int s = 0; s < NS; ++s)
                     if (issued & (1u << s)) mbar_wait_bounded(&ctl.full[s], (issued_par >> s) & 1u);

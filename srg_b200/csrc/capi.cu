@@ -358,6 +358,11 @@ StreamValueOps stream_value_ops() {
     return ops;
 }
 
+// The lines' base and row stride suit a TMA descriptor (16-byte units).
+static bool tma_lines(const BurstDev &B) {
+    return !(reinterpret_cast<uintptr_t>(B.burst) & 15) && !((B.ldb * 8) & 15) && !(B.bin0 & 1);
+}
+
 // Kernel entry for a form and shape index (-1: the default of that form).
 const KernelEntry *pick_kernel(int form, int cfg) {
     if (cfg >= 0) {
@@ -367,6 +372,31 @@ const KernelEntry *pick_kernel(int form, int cfg) {
     for (int i = 0; i < kNumKernels; ++i)
         if (kKernels[i].form == form) return &kKernels[i];
     return nullptr;
+}
+
+// The default shape of a launch over n bursts (KernelEntry order decides
+// elsewhere).  The split form's first shape stages 128 range bins; a 32 x 8
+// tile's pixels spread over |bins per column| 31 + |bins per line| 7 of them on
+// flat earth, and 8 go to the window's margins.  Beyond that nearly every
+// chunk takes the general path, so such grids (more than about 3.3 bins per
+// column: coarse pixels, oversampled lines) get the twin of that shape with
+// wide stages, whose results are the same; so do lines that have no TMA
+// descriptor (odd row strides), which the twin stages asynchronously (1,500
+// pulses of 21,001 samples: 1.3 ms, 7.7 in the first shape).  kFlat leaves room
+// for the relief inside a tile; below it the twin costs up to 1 %.
+const KernelEntry *pick_default(int form, int cfg, const srg_burst_desc *descs, int n) {
+    const KernelEntry *ke = pick_kernel(form, cfg);
+    if (!ke || cfg >= 0 || form != SRG_FORM_SPLIT) return ke;
+    constexpr double kFlat = 112.0;
+    for (int i = 0; i < n; ++i) {
+        const BurstDev B = make_burst_dev(descs[i], nullptr);
+        const double need = std::fabs(B.rbin_col) * (ke->shape.tx - 1) +
+                            std::fabs(B.rbin_line) * (ke->shape.ty - 1) + 8.0;
+        if (!(need > kFlat) && tma_lines(B)) continue;
+        for (int k = 0; k < kNumKernels; ++k)
+            if (kKernels[k].form == form && kKernels[k].wide) return &kKernels[k];
+    }
+    return ke;
 }
 
 // Reference line/pixel limits (azimuth_compress.cu:295-301, 378-379).
@@ -584,8 +614,7 @@ int set_tiles(BurstDev &B, const KernelEntry &ke, int shear) {
 int make_tmap(const BurstDev &B, int box_x, int box_y, CUtensorMap *out) {
     auto enc = get_encode();
     if (!enc) return -1;
-    const uintptr_t base = reinterpret_cast<uintptr_t>(B.burst);
-    if ((base & 15) || ((B.ldb * 8) & 15) || (box_x & 1) || (B.bin0 & 1)) return -1;
+    if ((box_x & 1) || !tma_lines(B)) return -1;
     cuuint64_t dims[2] = {(cuuint64_t)B.nbins, (cuuint64_t)B.P};
     cuuint64_t strides[1] = {(cuuint64_t)(B.ldb * 8)};
     cuuint32_t box[2] = {(cuuint32_t)box_x, (cuuint32_t)box_y};
@@ -594,6 +623,11 @@ int make_tmap(const BurstDev &B, int box_x, int box_y, CUtensorMap *out) {
                      estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? 0 : -1;
+}
+
+int make_tmaps(const BurstDev &B, const KernelEntry &ke, CUtensorMap *one, CUtensorMap *wide) {
+    if (make_tmap(B, ke.shape.window, ke.shape.chunk, one)) return -1;
+    return ke.wide ? make_tmap(B, kWideBins, kWideRows, wide) : 0;
 }
 
 // Device line centres for one descriptor into `coef` (device).
@@ -727,28 +761,30 @@ int run_bursts(DevCtx &c, const srg_burst_desc *descs, int n, const srg_bp_optio
                cudaStream_t st, cudaEvent_t before_sum = nullptr,
                const UploadGate *gate = nullptr, int *band = nullptr, int *band_host = nullptr,
                cudaEvent_t band_ready = nullptr) {
-    const KernelEntry *ke = pick_kernel(o.form, o.tile_cfg);
+    for (int i = 0; i < n; ++i) {
+        const int rc = validate_desc(descs[i]);
+        if (rc) return rc;
+    }
+    const KernelEntry *ke = gate ? pick_kernel(o.form, o.tile_cfg)
+                                 : pick_default(o.form, o.tile_cfg, descs, n);
     if (!ke) return fail(SRG_E_ARG, "no kernel for form %d shape %d", o.form, o.tile_cfg);
     const KernelEntry *twin = gate && n == 1 ? gated_twin(*ke) : nullptr;
     const bool gated = twin != nullptr;
     const int TX = ke->shape.tx, TY = ke->shape.ty;
     // coefficient scratch
     size_t coef_total = 0;
-    for (int i = 0; i < n; ++i) {
-        int rc = validate_desc(descs[i]);
-        if (rc) return rc;
+    for (int i = 0; i < n; ++i)
         if (!descs[i].coef) coef_total += 3 * (size_t)descs[i].nlines;
-    }
     int rc = c.coef.ensure(sizeof(double) * std::max<size_t>(coef_total, 3));
     if (rc) return rc;
     rc = c.bursts.ensure(sizeof(BurstDev) * n);
     if (rc) return rc;
-    rc = c.tmaps.ensure(sizeof(CUtensorMap) * n);
+    rc = c.tmaps.ensure(sizeof(CUtensorMap) * 2 * n);
     if (rc) return rc;
     rc = c.flags.ensure(64);
     if (rc) return rc;
     std::vector<BurstDev> hb(n);
-    std::vector<CUtensorMap> hm(n);
+    std::vector<CUtensorMap> hm(2 * (size_t)n);
     double *coef_base = static_cast<double *>(c.coef.p);
     size_t coef_off = 0;
     int total = 0, max_burst_tiles = 0;
@@ -773,7 +809,7 @@ int run_bursts(DevCtx &c, const srg_burst_desc *descs, int n, const srg_bp_optio
         B.tile_base = total;
         total += B.tiles_x * B.tiles_y;
         max_burst_tiles = std::max(max_burst_tiles, B.tiles_x * B.tiles_y);
-        if (make_tmap(B, ke->shape.window, ke->shape.chunk, &hm[i]) == 0) B.tmap = i;
+        if (make_tmaps(B, *ke, &hm[i], &hm[n + i]) == 0) B.tmap = i;
         if (gated) {
             B.ready = gate->word;
             B.ready_base = gate->base;
@@ -794,7 +830,7 @@ int run_bursts(DevCtx &c, const srg_burst_desc *descs, int n, const srg_bp_optio
     rc = c.tiles.ensure(tile_list_bytes(total));
     if (rc) return rc;
     CK(cudaMemcpyAsync(c.bursts.p, hb.data(), sizeof(BurstDev) * n, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(c.tmaps.p, hm.data(), sizeof(CUtensorMap) * n, cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(c.tmaps.p, hm.data(), sizeof(CUtensorMap) * hm.size(), cudaMemcpyHostToDevice, st));
     CK(cudaMemsetAsync(c.flags.p, 0, sizeof(int), st));  // work counter only
     const int idx = kernel_index(ke);
     ensure_attrs(c, idx);
@@ -866,7 +902,7 @@ int srg_tile_config_count(void) { return kNumKernels; }
 int srg_tile_shear(const srg_burst_desc *b, int tile_cfg, int tile_shear, int *shear,
                    int *tiles_x, int *tiles_y) {
     if (!b || !shear || !tiles_x || !tiles_y) return fail(SRG_E_ARG, "null argument");
-    const KernelEntry *ke = tile_cfg < 0 ? pick_kernel(SRG_FORM_SPLIT, -1)
+    const KernelEntry *ke = tile_cfg < 0 ? pick_default(SRG_FORM_SPLIT, -1, b, 1)
                             : tile_cfg < kNumKernels ? &kKernels[tile_cfg] : nullptr;
     if (!ke) return fail(SRG_E_ARG, "shape index %d", tile_cfg);
     BurstDev B = make_burst_dev(*b, nullptr);

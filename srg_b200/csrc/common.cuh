@@ -9,6 +9,10 @@ namespace srg {
 // suspending up to ~1 us; a launch may set another through BurstDev::spin).
 constexpr unsigned kSpinLimit = 1u << 22;
 
+// Stages of a wide chunk: bins and pulses (30,720 bytes; 31 pulses by 128 bins
+// hold 31,744).
+constexpr int kWideRows = 16, kWideBins = 240;
+
 // Error bits raised by kernels into the device error word.
 enum : int {
     ERR_TMA_TIMEOUT = 1,   // a bounded mbarrier wait for a TMA tile gave up

@@ -111,6 +111,9 @@ StreamValueOps stream_value_ops();
 int ensure_dropin(DevCtx &c);
 // Kernel entry for a form and shape index (-1: the default of that form).
 const KernelEntry *pick_kernel(int form, int cfg);
+// The same for a launch over the given (valid) bursts: the default takes their
+// geometry into account.
+const KernelEntry *pick_default(int form, int cfg, const srg_burst_desc *descs, int n);
 int kernel_index(const KernelEntry *e);
 void ensure_attrs(DevCtx &c, int idx);
 int validate_desc(const srg_burst_desc &d);
@@ -123,6 +126,8 @@ BurstDev make_burst_dev(const srg_burst_desc &d, const double *coef);
 int set_tiles(BurstDev &B, const KernelEntry &ke, int shear);
 // 0 and *out filled when a TMA descriptor can describe the burst, else -1.
 int make_tmap(const BurstDev &B, int box_x, int box_y, CUtensorMap *out);
+// make_tmap for the box of `ke` and, where its tiles may widen, for the wide one.
+int make_tmaps(const BurstDev &B, const KernelEntry &ke, CUtensorMap *one, CUtensorMap *wide);
 double ref_pi();
 // |x - s_k|^2 is convex in the pulse index k for every pixel x that can have
 // a term in range (the range band's bisection relies on it).

@@ -516,6 +516,10 @@ cudaError_t launch_fma_peak(int fp64, int blocks, int iters, void *sink, cudaStr
     X(FORM_SPLIT, 16, 16, 4, 31, 2, 128, 3)  \
     X(FORM_SPLIT, 32, 8, 4, 16, 2, 256, 3)
 
+// Shapes that stage a chunk in two wide windows where its pixels need it (bp_ws:
+// WIDE).
+#define SRG_WIDE_SHAPES(X) X(FORM_SPLIT, 32, 8, 4, 31, 2, 128, 3)
+
 #define SRG_WS_FP64_SHAPES(X)               \
     X(FORM_FP64, 32, 4, 4, 16, 2, 128, 3)   \
     X(FORM_FP64, 32, 8, 4, 16, 2, 128, 2)
@@ -523,17 +527,23 @@ cudaError_t launch_fma_peak(int fp64, int blocks, int iters, void *sink, cudaStr
 #define SRG_ENTRY(F, TXv, TYv, NTv, CKv, WBv)                                                   \
     {F, {TXv, TYv, NTv, CKv, WBv}, params_bytes<F, CKv>() + 1024 + CKv * WBv * 8,               \
      (const void *)bp_tiles<F, TXv, TYv, NTv, CKv>,                                             \
-     "bp_tiles<" #F "," #TXv "x" #TYv ",threads " #NTv ",chunk " #CKv ",window " #WBv ">", 0},
+     "bp_tiles<" #F "," #TXv "x" #TYv ",threads " #NTv ",chunk " #CKv ",window " #WBv ">", 0, 0},
 #define SRG_WS_ENTRY(F, TXv, TYv, NCv, CKv, NSv, WBv, MBv)                                      \
     {F, {TXv, TYv, (NCv + 1) * 32, CKv, WBv}, ws_smem_bytes<F, CKv, NSv>(WBv),                  \
      (const void *)bp_ws<F, TXv, TYv, NCv, CKv, NSv, WBv, MBv>,                                 \
      "bp_ws<" #F "," #TXv "x" #TYv ",consumer warps " #NCv ",chunk " #CKv ",stages " #NSv       \
-     ",window " #WBv ",min blocks " #MBv ">", 1},
+     ",window " #WBv ",min blocks " #MBv ">", 1, 0},
+#define SRG_WIDE_ENTRY(F, TXv, TYv, NCv, CKv, NSv, WBv, MBv)                                    \
+    {F, {TXv, TYv, (NCv + 1) * 32, CKv, WBv}, ws_smem_bytes<F, CKv, NSv>(WBv),                  \
+     (const void *)bp_ws<F, TXv, TYv, NCv, CKv, NSv, WBv, MBv, false, true>,                    \
+     "bp_ws<" #F "," #TXv "x" #TYv ",consumer warps " #NCv ",chunk " #CKv ",stages " #NSv       \
+     ",window " #WBv " or wide,min blocks " #MBv ">", 1, 1},
 
 // The first shape of a form is its default: the fastest measured on the
 // B200 (warp-specialised for the split form, first generation for FP64).
 const KernelEntry kKernels[] = {SRG_WS_SHAPES(SRG_WS_ENTRY) SRG_SHAPES(SRG_ENTRY)
-                                    SRG_WS_FP64_SHAPES(SRG_WS_ENTRY)};
+                                    SRG_WS_FP64_SHAPES(SRG_WS_ENTRY)
+                                    SRG_WIDE_SHAPES(SRG_WIDE_ENTRY)};
 const int kNumKernels = sizeof(kKernels) / sizeof(kKernels[0]);
 
 // Gated twins (range lines still uploading; the drop-in entry) of the
@@ -542,7 +552,7 @@ const int kNumKernels = sizeof(kKernels) / sizeof(kKernels[0]);
     {F, {TXv, TYv, (NCv + 1) * 32, CKv, WBv}, ws_smem_bytes<F, CKv, NSv>(WBv),                  \
      (const void *)bp_ws<F, TXv, TYv, NCv, CKv, NSv, WBv, MBv, true>,                           \
      "bp_ws<" #F "," #TXv "x" #TYv ",consumer warps " #NCv ",chunk " #CKv ",stages " #NSv       \
-     ",window " #WBv ",min blocks " #MBv ",gated>", 1},
+     ",window " #WBv ",min blocks " #MBv ",gated>", 1, 0},
 const KernelEntry kGatedKernels[] = {SRG_WS_GATED_ENTRY(FORM_SPLIT, 32, 8, 4, 31, 2, 128, 3)};
 const int kNumGatedKernels = sizeof(kGatedKernels) / sizeof(kGatedKernels[0]);
 

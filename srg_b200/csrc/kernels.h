@@ -28,6 +28,8 @@ struct KernelEntry {
     const void *fn;
     const char *name;  // template and shape, for reports
     int shears;        // 1: the kernel takes sheared tiles (BurstDev::shear)
+    int wide;          // 1: wide chunks use a second TMA descriptor, at tmaps[bursts + burst],
+                       // of a box of kWideBins x kWideRows
 };
 
 extern const KernelEntry kKernels[];

@@ -31,12 +31,13 @@ constexpr int kMaxLines = SRG_NOALLOC_MAX_LINES;
 constexpr int kMaxStateVec = SRG_NOALLOC_MAX_STATEVEC;
 constexpr size_t kOffFlags = 0;        // int work counter, int error word
 constexpr size_t kOffBurst = 256;      // BurstDev
-constexpr size_t kOffTmap = 1024;      // CUtensorMap (64-byte aligned)
+constexpr size_t kOffTmap = 1024;      // CUtensorMap [2] (64-byte aligned)
 constexpr size_t kOffOrbit = 2048;     // [n] times, [n][3] positions, [n][3] velocities
 constexpr size_t kOffCoef = kOffOrbit + 7 * sizeof(double) * kMaxStateVec;
 constexpr size_t kScratchBytes = kOffCoef + 3 * sizeof(double) * kMaxLines;
 static_assert(kScratchBytes == SRG_NOALLOC_SCRATCH_BYTES, "header and layout disagree");
 static_assert(sizeof(BurstDev) <= kOffTmap - kOffBurst, "BurstDev outgrew its slot");
+static_assert(2 * sizeof(CUtensorMap) <= kOffOrbit - kOffTmap, "descriptors outgrew their slot");
 static_assert(kOffTmap % 64 == 0 && kOffCoef % 8 == 0, "alignment");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
@@ -78,7 +79,7 @@ extern "C" int srg_bp_burst_device_noalloc(const srg_burst_desc *b, const srg_bp
     if (opts) o = *opts;
     if (o.centres_on_host && !b->coef)  // as srg_bp_bursts_device
         return fail(SRG_E_UNSUPPORTED, "host centres need host DEM (use the file entry)");
-    const KernelEntry *ke = pick_kernel(o.form, o.tile_cfg);
+    const KernelEntry *ke = pick_default(o.form, o.tile_cfg, b, 1);
     if (!ke) return fail(SRG_E_ARG, "no kernel for form %d shape %d", o.form, o.tile_cfg);
     DevCtx *c = nullptr;
     rc = get_ctx(o.device, &c);
@@ -131,11 +132,11 @@ extern "C" int srg_bp_burst_device_noalloc(const srg_burst_desc *b, const srg_bp
     if ((rc = set_tiles(B, *ke, o.tile_shear))) return rc;
     B.tile_base = 0;
     const int total = B.tiles_x * B.tiles_y;
-    CUtensorMap tm;
-    std::memset(&tm, 0, sizeof tm);
-    if (make_tmap(B, ke->shape.window, ke->shape.chunk, &tm) == 0) B.tmap = 0;
+    CUtensorMap tm[2];
+    std::memset(tm, 0, sizeof tm);
+    if (make_tmaps(B, *ke, &tm[0], &tm[1]) == 0) B.tmap = 0;
     NA_CK(cudaMemcpyAsync(d_burst, &B, sizeof B, cudaMemcpyHostToDevice, st));
-    NA_CK(cudaMemcpyAsync(d_tmap, &tm, sizeof tm, cudaMemcpyHostToDevice, st));
+    NA_CK(cudaMemcpyAsync(d_tmap, tm, sizeof tm, cudaMemcpyHostToDevice, st));
     if (total > 0) {
         const int idx = kernel_index(ke);
         ensure_attrs(*c, idx);

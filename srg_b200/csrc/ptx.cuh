@@ -130,6 +130,21 @@ __device__ __forceinline__ bool wait_word_at_least(const int *word, int target,
     return ok != 0;
 }
 
+// Asynchronous copy of one complex64 sample from global to shared memory; zeros
+// where !use (nothing is read then).
+__device__ __forceinline__ void cp_async_sample(float2 *dst, const float2 *src, bool use) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src),
+                 "r"(use ? 8 : 0)
+                 : "memory");
+}
+// One more arrival on `bar`'s current phase, made when this thread's copies so
+// far have landed (the phase's own count is unchanged).
+__device__ __forceinline__ void cp_async_arrive(uint64_t *bar) {
+    asm volatile("cp.async.mbarrier.arrive.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// Waits for this thread's copies.
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // 2D tiled TMA load of box {box_x, box_y} at element coordinates (x, y) into
 // shared memory, completing on `bar` (byte count set by the caller).  The
 // tensor map lives in global memory, written by the host before launch.

@@ -93,7 +93,7 @@ void drop_graph(srg_scene *s) {
 // (Re)build the burst table and TMA descriptors for kernel shape `idx`.
 int set_kernel(srg_scene *s, int idx) {
     const KernelEntry &ke = kKernels[idx];
-    std::vector<CUtensorMap> hm(s->n);
+    std::vector<CUtensorMap> hm(2 * (size_t)s->n);
     int total = 0, max_burst_tiles = 0;
     for (int i = 0; i < s->n; ++i) {
         BurstDev &B = s->hb[i];
@@ -102,7 +102,8 @@ int set_kernel(srg_scene *s, int idx) {
         total += B.tiles_x * B.tiles_y;
         max_burst_tiles = std::max(max_burst_tiles, B.tiles_x * B.tiles_y);
         std::memset(&hm[i], 0, sizeof(CUtensorMap));
-        B.tmap = make_tmap(B, ke.shape.window, ke.shape.chunk, &hm[i]) == 0 ? i : -1;
+        std::memset(&hm[s->n + i], 0, sizeof(CUtensorMap));
+        B.tmap = make_tmaps(B, ke, &hm[i], &hm[s->n + i]) == 0 ? i : -1;
     }
     // An earlier pass of the plan may still read the descriptors on a caller's
     // non-blocking stream, which the legacy stream's copies below do not wait
@@ -110,7 +111,7 @@ int set_kernel(srg_scene *s, int idx) {
     // may still be in flight when cudaMemcpy returns: wait for them too.
     SCK(cudaDeviceSynchronize());
     SCK(cudaMemcpy(s->d_bursts, s->hb.data(), sizeof(BurstDev) * s->n, cudaMemcpyHostToDevice));
-    SCK(cudaMemcpy(s->d_tmaps, hm.data(), sizeof(CUtensorMap) * s->n, cudaMemcpyHostToDevice));
+    SCK(cudaMemcpy(s->d_tmaps, hm.data(), sizeof(CUtensorMap) * hm.size(), cudaMemcpyHostToDevice));
     SCK(cudaStreamSynchronize(0));
     const size_t need = tile_list_bytes(total);
     if (need > s->tiles_cap) {
@@ -142,6 +143,14 @@ srg_burst_desc kernel_desc(const srg_scene *s, int i) {
         d.bin0 = d.nbins = 0;
     }
     return d;
+}
+
+// The kernel of a form and shape index on the plan's bursts as the kernels see
+// them (-1: the default for their geometry), or null.
+const KernelEntry *choose_kernel(const srg_scene *s, int form, int cfg) {
+    std::vector<srg_burst_desc> d(s->n);
+    for (int i = 0; i < s->n; ++i) d[i] = kernel_desc(s, i);
+    return pick_default(form, cfg, d.data(), s->n);
 }
 
 // The 2x oversampling of every burst's lines into the plan's copies.
@@ -213,6 +222,8 @@ int rebuild_bursts(srg_scene *s) {
         s->hb[i].spin = spin;
     }
     s->terms = -1;
+    if (s->opts.tile_cfg < 0)  // no shape asked for: the default for the lines in use
+        return set_kernel(s, kernel_index(choose_kernel(s, s->opts.form, -1)));
     return set_kernel(s, s->kernel);
 }
 
@@ -311,8 +322,8 @@ int srg_scene_create(const srg_burst_desc *bursts, int n, float *scene, int64_t 
     srg_bp_options o;
     srg_bp_default_options(&o);
     if (opts) o = *opts;
-    const KernelEntry *ke = pick_kernel(o.form, o.tile_cfg);
-    if (!ke) return fail(SRG_E_ARG, "no kernel for form %d shape %d", o.form, o.tile_cfg);
+    if (!pick_kernel(o.form, o.tile_cfg))
+        return fail(SRG_E_ARG, "no kernel for form %d shape %d", o.form, o.tile_cfg);
     for (int i = 0; i < n; ++i) {
         int rc = validate_desc(bursts[i]);
         if (rc) return rc;
@@ -321,6 +332,7 @@ int srg_scene_create(const srg_burst_desc *bursts, int n, float *scene, int64_t 
         if (bursts[i].numstatevec < 4 || bursts[i].numstatevec > 4096)
             return fail(SRG_E_ARG, "burst %d: numstatevec %d", i, bursts[i].numstatevec);
     }
+    const KernelEntry *ke = pick_default(o.form, o.tile_cfg, bursts, n);
     DevCtx *c = nullptr;
     int rc = get_ctx(o.device, &c);
     if (rc) return rc;
@@ -339,7 +351,7 @@ int srg_scene_create(const srg_burst_desc *bursts, int n, float *scene, int64_t 
         orbit += 7 * (size_t)bursts[i].numstatevec;
     }
     if ((rc = alloc((void **)&s->d_bursts, sizeof(BurstDev) * n)) ||
-        (rc = alloc((void **)&s->d_tmaps, sizeof(CUtensorMap) * n)) ||
+        (rc = alloc((void **)&s->d_tmaps, sizeof(CUtensorMap) * 2 * n)) ||
         (rc = alloc((void **)&s->d_jobs, sizeof(CentreJob) * n)) ||
         (rc = alloc((void **)&s->d_coef, sizeof(double) * 3 * lines)) ||
         (rc = alloc((void **)&s->d_orbit, sizeof(double) * orbit)) ||
@@ -612,7 +624,7 @@ int srg_scene_interp(const srg_scene *s) { return s ? s->interp : -1; }
 
 int srg_scene_set_shape(srg_scene *s, int tile_cfg) {
     if (!s) return fail(SRG_E_ARG, "null plan");
-    const KernelEntry *ke = pick_kernel(s->opts.form, tile_cfg);
+    const KernelEntry *ke = choose_kernel(s, s->opts.form, tile_cfg);
     if (!ke) return fail(SRG_E_ARG, "no kernel for form %d shape %d", s->opts.form, tile_cfg);
     s->opts.tile_cfg = tile_cfg;
     return set_kernel(s, kernel_index(ke));
@@ -620,7 +632,7 @@ int srg_scene_set_shape(srg_scene *s, int tile_cfg) {
 
 int srg_scene_set_form(srg_scene *s, int form, int tile_cfg) {
     if (!s) return fail(SRG_E_ARG, "null plan");
-    const KernelEntry *ke = pick_kernel(form, tile_cfg);
+    const KernelEntry *ke = choose_kernel(s, form, tile_cfg);
     if (!ke) return fail(SRG_E_ARG, "no kernel for form %d shape %d", form, tile_cfg);
     s->opts.form = form;
     s->opts.tile_cfg = tile_cfg;
