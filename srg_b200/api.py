@@ -377,6 +377,17 @@ def range_replica(samplefreq: float, startfreq: float, ramprate: float, pulselen
     return rep, int(npts.value)
 
 
+def _replica_points(samplefreq, startfreq, ramprate, pulselength) -> int:
+    """npts of ``range_replica`` without making the replica: the pulse length
+    times the sampling rate in single precision, truncated (0.2 ms of sines per
+    call otherwise).  What the library refuses goes to it for the error."""
+    with np.errstate(over="ignore"):
+        prod = np.float32(pulselength) * np.float32(samplefreq)
+    if samplefreq > 0 and pulselength > 0 and 1 <= prod < 32769:
+        return int(prod)
+    return range_replica(samplefreq, startfreq, ramprate, pulselength)[1]
+
+
 def range_compress(lines, samplefreq: float, startfreq: float, ramprate: float, pulselength: float,
                    nsamps: Optional[int] = None, out=None, stream=None, sync: bool = True):
     """Range-compress decoded echo lines (complex64 CUDA tensor [nlines][>= nsamps],
@@ -388,7 +399,7 @@ def range_compress(lines, samplefreq: float, startfreq: float, ramprate: float, 
         raise ValueError("lines must be a 2-D complex64 CUDA tensor with unit column stride")
     nlines = lines.shape[0]
     nsamps = lines.shape[1] if nsamps is None else nsamps
-    _, npts = range_replica(samplefreq, startfreq, ramprate, pulselength)
+    npts = _replica_points(samplefreq, startfreq, ramprate, pulselength)
     nvalid = nsamps - npts
     if out is None:
         out = torch.empty((nlines, max(nvalid, 1)), dtype=torch.complex64, device=lines.device)

@@ -186,6 +186,17 @@ struct RcCtx {
 };
 RcCtx g_rc[64];
 
+// Samples of the replica of a pulse (processsub.f90:94), and whether n hold them.
+int replica_points(float samplefreq, float pulselength, int n, int *npts) {
+    if (n < 1 || !(samplefreq > 0) || !(pulselength > 0))
+        return fail(SRG_E_ARG, "bad replica arguments");
+    const float prod = pulselength * samplefreq;  // real*4 product
+    *npts = (int)prod;                            // truncated, as the Fortran assignment
+    if (*npts < 1 || *npts > n)
+        return fail(SRG_E_ARG, "replica of %d samples does not fit %d", *npts, n);
+    return SRG_OK;
+}
+
 int grid_of(long long n) { return (int)std::min<long long>((n + 255) / 256, 148LL * 32); }
 
 }  // namespace
@@ -194,12 +205,10 @@ extern "C" {
 
 int srg_range_replica(float samplefreq, float startfreq, float ramprate, float pulselength,
                       float *replica, int n, int *npts_out) {
-    if (!replica || n < 1 || !(samplefreq > 0) || !(pulselength > 0))
-        return fail(SRG_E_ARG, "bad replica arguments");
+    if (!replica) return fail(SRG_E_ARG, "bad replica arguments");
+    int npts = 0;
+    if (const int rc = replica_points(samplefreq, pulselength, n, &npts)) return rc;
     const double pi = 4.0 * std::atan2(1.0, 1.0);
-    const float prod = pulselength * samplefreq;  // real*4 product
-    const int npts = (int)prod;                   // truncated, as the Fortran assignment
-    if (npts < 1 || npts > n) return fail(SRG_E_ARG, "replica of %d samples does not fit %d", npts, n);
     std::memset(replica, 0, sizeof(float) * 2 * (size_t)n);
     for (int j = 1; j <= npts; ++j) {
         const double t = (double)((float)(j - 1) / samplefreq);
@@ -217,9 +226,8 @@ int srg_range_compress_device(const float *lines, long long ld_in, int nlines, i
     if (!lines || !out || nlines < 1 || nsamps < 1 || nsamps > kRangeFFT || ld_in < nsamps)
         return fail(SRG_E_ARG, "bad range-compression sizes: nlines=%d nsamps=%d (<= %d) ld=%lld",
                     nlines, nsamps, kRangeFFT, ld_in);
-    std::vector<float> rep(2 * (size_t)kRangeFFT);
     int npts = 0;
-    int rc = srg_range_replica(samplefreq, startfreq, ramprate, pulselength, rep.data(), kRangeFFT, &npts);
+    int rc = replica_points(samplefreq, pulselength, kRangeFFT, &npts);
     if (rc) return rc;
     const int nvalid = nsamps - npts;
     if (nvalid < 1) return fail(SRG_E_ARG, "pulse of %d samples leaves no valid sample of %d", npts, nsamps);
@@ -252,6 +260,10 @@ int srg_range_compress_device(const float *lines, long long ld_in, int nlines, i
         if (std::memcmp(key, x.os_key, sizeof key) != 0) {
             // H = (32768 / 8192) conj(DFT_8192(replica)), in FP64 from the
             // replica's complex64 samples
+            std::vector<float> rep(2 * (size_t)kOsM);
+            if ((rc = srg_range_replica(samplefreq, startfreq, ramprate, pulselength, rep.data(), kOsM,
+                                        &npts)))
+                return rc;
             std::vector<std::complex<double>> a(kOsM);
             for (int j = 0; j < npts; ++j) a[j] = std::complex<double>(rep[2 * j], rep[2 * j + 1]);
             host_fft(a);
@@ -288,6 +300,10 @@ int srg_range_compress_device(const float *lines, long long ld_in, int nlines, i
     const float key[4] = {samplefreq, startfreq, ramprate, pulselength};
     if (std::memcmp(key, x.key, sizeof key) != 0) {
         // replica spectrum (processsub.f90:101-108)
+        std::vector<float> rep(2 * (size_t)kRangeFFT);
+        if ((rc = srg_range_replica(samplefreq, startfreq, ramprate, pulselength, rep.data(), kRangeFFT,
+                                    &npts)))
+            return rc;
         CKR(cudaMemcpyAsync(ref, rep.data(), sizeof(float2) * kRangeFFT, cudaMemcpyHostToDevice, st));
         CKFR(cufftSetStream(x.plan_one, st));
         CKFR(cufftExecC2C(x.plan_one, reinterpret_cast<cufftComplex *>(ref),
