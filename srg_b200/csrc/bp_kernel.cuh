@@ -43,6 +43,7 @@
 #pragma once
 #include <climits>
 #include <cuda.h>
+#include <type_traits>
 #include "common.cuh"
 #include "geom.cuh"
 #include "ptx.cuh"
@@ -131,6 +132,79 @@ __device__ __forceinline__ float2 ld_sample(const BurstDev &B, int k, int gi) {
     if (gi >= 0 && gi < B.S && (unsigned)p < (unsigned)B.nbins && k < B.P)
         return __ldg(B.burst + (long long)k * B.ldb + p);
     return make_float2(0.f, 0.f);
+}
+
+// *p where `use`, else `v`, without a branch.
+__device__ __forceinline__ float2 ld_where(bool use, const float2 *p, float2 v) {
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\t"
+        "@q ld.global.nc.v2.f32 {%0, %1}, [%3];\n\t}"
+        : "+f"(v.x), "+f"(v.y)
+        : "r"((int)use), "l"(p));
+    return v;
+}
+
+// ---- FP64 steps of a term ----
+// x / d correctly rounded, for a divisor whose correctly rounded reciprocal
+// inv is at hand (d: the burst's bin spacing): x inv is within two units in the
+// last place of the quotient, one residual step (exact remainder by FMA, then
+// times inv) makes it faithful and the second one correct (Markstein, "Computation
+// of elementary functions on the IBM RISC System/6000", 1990).  Five operations
+// without a branch, the same bits as the division.
+__device__ __forceinline__ double div_by(double x, double d, double inv) {
+    double q = x * inv;
+    q = fma(fma(-q, d, x), inv, q);
+    return fma(fma(-q, d, x), inv, q);
+}
+
+// sqrt(x) correctly rounded, x a positive normal number: from the hardware's
+// reciprocal square root (20 bits) two coupled Newton steps for sqrt(x) and
+// 1 / (2 sqrt(x)), then one residual step with the exact remainder (Markstein,
+// "IA-64 and elementary functions", 2000).  Eleven operations and no branch, the
+// same bits as the correctly rounded function.
+__device__ __forceinline__ double sqrt_pos(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    double g = x * y, h = 0.5 * y;
+    double r = fma(-g, h, 0.5);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    r = fma(-g, h, 0.5);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    return fma(fma(-g, g, x), h, g);
+}
+
+// sin and cos of x, 0 <= x < 2^30, within one unit in the last place: x less
+// the nearest multiple n of pi/2 in two parts (Cody and Waite; the first
+// product and difference are exact in an FMA: x has no bits below 2^-23 that
+// pi/2's do not reach, and the remainder is below 1), then polynomials through
+// the Chebyshev points of the interval (interpolated in rational arithmetic;
+// errors 1.8e-17 and 9e-19).  24 FP64 operations and no branch.
+constexpr double kSinCosMax = 1073741824.0;
+__device__ __forceinline__ void sincos_pos(double x, double *sn, double *cs) {
+    const double magic = 6755399441055744.0;  // 1.5 * 2^52: rounds to an integer in the low word
+    const double m = fma(x, 0.63661977236758138, magic);
+    const int q = __double2loint(m);
+    const double n = m - magic;
+    const double r = fma(n, -6.123233995736766e-17, fma(n, -1.5707963267948966, x));
+    const double z = r * r;
+    double s = fma(z, 1.5917848524808262e-10, -2.5051127944014188e-08);
+    s = fma(z, s, 2.755731608381636e-06);
+    s = fma(z, s, -0.00019841269836722418);
+    s = fma(z, s, 0.008333333333330925);
+    s = fma(z, s, -0.16666666666666666);
+    s = fma(z * r, s, r);
+    double c = fma(z, -1.1382456778061306e-11, 2.0876143827993133e-09);
+    c = fma(z, c, -2.7557317260008837e-07);
+    c = fma(z, c, 2.480158729874307e-05);
+    c = fma(z, c, -0.0013888888888887382);
+    c = fma(z, c, 0.041666666666666664);
+    c = fma(z, c, -0.5);
+    c = fma(z, c, 1.0);
+    // quarter turns: swap, then the signs, on the words
+    const double a = q & 1 ? c : s, b = q & 1 ? s : c;
+    *sn = __hiloint2double(__double2hiint(a) ^ ((q << 30) & 0x80000000), __double2loint(a));
+    *cs = __hiloint2double(__double2hiint(b) ^ (((q + 1) << 30) & 0x80000000), __double2loint(b));
 }
 
 // Stages pulses [k0, k0 + rows) x bins [x0, x0 + wb) of a burst without a TMA
@@ -452,42 +526,74 @@ bp_tiles(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
 #pragma unroll
                 for (int m = 0; m < M; ++m) c[m] -= rintf(c[m]);
             } else {
-                const double rs = B.rngstart, rmax = B.rmax, dm = B.dmrg, k4 = B.k4pi;
-                for (int j = 0; j < nk; ++j) {
-                    const int k = k0 + j;
-                    const double sx = prmd[4 * j + 0], sy = prmd[4 * j + 1], sz = prmd[4 * j + 2];
-                    const float2 *row = samp + j * WB;
+                const double rs = B.rngstart, rmax = B.rmax, dm = B.dmrg, idm = B.inv_dmrg, k4 = B.k4pi;
+                // the pixels' windows within the chunk
+                int ja[M], nj[M];
 #pragma unroll
-                    for (int m = 0; m < M; ++m) {
-                        if (k < azs[m] || k >= aze[m]) continue;
-                        const double vx = dsub(X[m][0], sx), vy = dsub(X[m][1], sy),
-                                     vz = dsub(X[m][2], sz);
-                        const double R = __dsqrt_rn(dadd(dadd(dmul(vx, vx), dmul(vy, vy)), dmul(vz, vz)));
-                        if (!(R >= rs && R <= rmax)) continue;
-                        const double r = ddiv(dsub(R, rs), dm);
-                        const double fl = floor(r);
-                        const int ig = (int)fl;
-                        const double fr = dsub(r, fl);
-                        const float w0 = __double2float_rn(dsub(1.0, fr));
-                        const float w1 = __double2float_rn(fr);
-                        const int i = ig - x0;
-                        float2 s0, s1;
-                        if ((unsigned)i < (unsigned)(WB - 1)) {
-                            s0 = row[i];
-                            s1 = row[i + 1];
-                        } else {
-                            s0 = ld_sample(B, k, ig);
-                            s1 = ld_sample(B, k, ig + 1);
-                        }
-                        const float cre = __fadd_rn(__fmul_rn(s0.x, w0), __fmul_rn(s1.x, w1));
-                        const float cim = __fadd_rn(__fmul_rn(s0.y, w0), __fmul_rn(s1.y, w1));
-                        double sn, cs;
-                        sincos(dmul(k4, R), &sn, &cs);
-                        const double a = (double)cre, bq = (double)cim;
-                        accr_d[m] += a * cs - bq * sn;
-                        acci_d[m] += a * sn + bq * cs;
-                    }
+                for (int m = 0; m < M; ++m) {
+                    ja[m] = max(azs[m] - k0, 0);
+                    nj[m] = max(min(aze[m] - k0, nk) - ja[m], 0);
                 }
+                // Two terms at a time (two pulses of a pixel, or one of two): a term
+                // is one dependent chain of about 54 FP64 operations, and the
+                // warps that fit (by shared memory) do not cover its latency.
+                // SMALL: every phase is below sincos_pos's limit.
+                auto terms = [&](auto small) {
+                    constexpr bool SMALL = decltype(small)::value;
+                    constexpr int U = M == 1 ? 2 : 1, E = M * U;
+                    for (int j = 0; j < nk; j += U) {
+                        double R[E];
+                        float2 s0[E], s1[E];
+                        float w0[E], w1[E];
+                        bool ok[E], any = false;
+#pragma unroll
+                        for (int e = 0; e < E; ++e) {
+                            // (pulse nk of an odd chunk: whatever the stage holds there, not ok)
+                            const int m = e % M, jj = j + e / M;
+                            const double vx = dsub(X[m][0], prmd[4 * jj + 0]),
+                                         vy = dsub(X[m][1], prmd[4 * jj + 1]),
+                                         vz = dsub(X[m][2], prmd[4 * jj + 2]);
+                            R[e] = sqrt_pos(dadd(dadd(dmul(vx, vx), dmul(vy, vy)), dmul(vz, vz)));
+                            ok[e] = ((unsigned)(jj - ja[m]) < (unsigned)nj[m]) & (R[e] >= rs) & (R[e] <= rmax);
+                            any |= ok[e];
+                        }
+                        if (!any) continue;
+#pragma unroll
+                        for (int e = 0; e < E; ++e) {
+                            const int jj = j + e / M;
+                            // r >= 0 where ok: its floor from an add rounded down
+                            const double r = div_by(dsub(R[e], rs), dm, idm);
+                            const double rm = __dadd_rd(r, 6755399441055744.0);
+                            const int ig = __double2loint(rm);
+                            const double fr = dsub(r, dsub(rm, 6755399441055744.0));
+                            w0[e] = __double2float_rn(dsub(1.0, fr));
+                            w1[e] = __double2float_rn(fr);
+                            const int i = ig - x0;
+                            const bool in = (unsigned)i < (unsigned)(WB - 1);
+                            const float2 *row = samp + jj * WB + (in ? i : 0);
+                            s0[e] = row[0];
+                            s1[e] = row[1];
+                            if (ok[e] & !in) {
+                                s0[e] = ld_sample(B, k0 + jj, ig);
+                                s1[e] = ld_sample(B, k0 + jj, ig + 1);
+                            }
+                        }
+#pragma unroll
+                        for (int e = 0; e < E; ++e) {
+                            const int m = e % M;
+                            const float cre = __fadd_rn(__fmul_rn(s0[e].x, w0[e]), __fmul_rn(s1[e].x, w1[e]));
+                            const float cim = __fadd_rn(__fmul_rn(s0[e].y, w0[e]), __fmul_rn(s1[e].y, w1[e]));
+                            double sn, cs;
+                            if constexpr (SMALL) sincos_pos(dmul(k4, R[e]), &sn, &cs);
+                            else sincos(dmul(k4, R[e]), &sn, &cs);
+                            const double a = (double)(ok[e] ? cre : 0.f), bq = (double)(ok[e] ? cim : 0.f);
+                            accr_d[m] = fma(-bq, sn, fma(a, cs, accr_d[m]));
+                            acci_d[m] = fma(bq, cs, fma(a, sn, acci_d[m]));
+                        }
+                    }
+                };
+                if (k4 * rmax < kSinCosMax) terms(std::true_type{});
+                else terms(std::false_type{});
             }
         }
 

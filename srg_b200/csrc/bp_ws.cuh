@@ -151,15 +151,6 @@ __device__ __forceinline__ unsigned tap_index(float tm) {
     else return min(__float_as_uint(tm) - (unsigned)kFloorMagicBits, (unsigned)(WB - 2));
 }
 
-// *p where `use`, else `v`, without a branch.
-__device__ __forceinline__ float2 ld_where(bool use, const float2 *p, float2 v) {
-    asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\t"
-        "@q ld.global.nc.v2.f32 {%0, %1}, [%3];\n\t}"
-        : "+f"(v.x), "+f"(v.y)
-        : "r"((int)use), "l"(p));
-    return v;
-}
-
 // Chunk schedule of a tile: the pulse range [kmin, kmax) is cut at ka and kb
 // (the interior segment [ka, kb) lies inside every formed pixel's aperture)
 // and each of the three segments into chunks of at most CK pulses, so that
@@ -1066,7 +1057,7 @@ bp_ws(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
                         cph[m] = fmaf(-nr, kTwoPiLo, fmaf(-nr, kTwoPiHi, cph[m]));
                     }
                 } else {
-                    const double rs = rng0_c, rmx = rmax_c, dm = dmrg_c, k4 = k4pi_c;
+                    const double rs = rng0_c, rmx = rmax_c, dm = dmrg_c, idm = B.inv_dmrg, k4 = k4pi_c;
                     const int x0 = h.x0;
                     const bool fast = h.fast && h.interior;
                     for (int j = 0; j < nk; ++j) {
@@ -1078,13 +1069,13 @@ bp_ws(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
                             if (!fast && (k < azs[m] || k >= aze[m])) continue;
                             const double vx = dsub(X[m][0], sx), vy = dsub(X[m][1], sy),
                                          vz = dsub(X[m][2], sz);
-                            const double R = __dsqrt_rn(dadd(dadd(dmul(vx, vx), dmul(vy, vy)), dmul(vz, vz)));
+                            const double R = sqrt_pos(dadd(dadd(dmul(vx, vx), dmul(vy, vy)), dmul(vz, vz)));
                             const bool inr = R >= rs && R <= rmx;
                             if (!fast && !inr) continue;
-                            const double rr = ddiv(dsub(R, rs), dm);
-                            const double fl = floor(rr);
-                            const int ig = (int)fl;
-                            const double fr = dsub(rr, fl);
+                            const double rr = div_by(dsub(R, rs), dm, idm);
+                            const double rm = __dadd_rd(rr, 6755399441055744.0);  // floor
+                            const int ig = __double2loint(rm);
+                            const double fr = dsub(rr, dsub(rm, 6755399441055744.0));
                             const float w0 = __double2float_rn(dsub(1.0, fr));
                             const float w1 = __double2float_rn(fr);
                             const int i = ig - x0;
@@ -1102,10 +1093,12 @@ bp_ws(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
                             const float cre = __fadd_rn(__fmul_rn(s0.x, w0), __fmul_rn(s1.x, w1));
                             const float cim = __fadd_rn(__fmul_rn(s0.y, w0), __fmul_rn(s1.y, w1));
                             double sn, cs;
-                            sincos(dmul(k4, R), &sn, &cs);
+                            const double ph = dmul(k4, R);
+                            if (ph < kSinCosMax) sincos_pos(ph, &sn, &cs);
+                            else sincos(ph, &sn, &cs);
                             const double a = (double)cre, bq = (double)cim;
-                            accr_d[m] += a * cs - bq * sn;
-                            acci_d[m] += a * sn + bq * cs;
+                            accr_d[m] = fma(-bq, sn, fma(a, cs, accr_d[m]));
+                            acci_d[m] = fma(bq, cs, fma(a, sn, acci_d[m]));
                         }
                     }
                 }
