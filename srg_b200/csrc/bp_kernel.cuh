@@ -144,18 +144,6 @@ __device__ __forceinline__ float2 ld_where(bool use, const float2 *p, float2 v) 
 }
 
 // ---- FP64 steps of a term ----
-// x / d correctly rounded, for a divisor whose correctly rounded reciprocal
-// inv is at hand (d: the burst's bin spacing): x inv is within two units in the
-// last place of the quotient, one residual step (exact remainder by FMA, then
-// times inv) makes it faithful and the second one correct (Markstein, "Computation
-// of elementary functions on the IBM RISC System/6000", 1990).  Five operations
-// without a branch, the same bits as the division.
-__device__ __forceinline__ double div_by(double x, double d, double inv) {
-    double q = x * inv;
-    q = fma(fma(-q, d, x), inv, q);
-    return fma(fma(-q, d, x), inv, q);
-}
-
 // sqrt(x) correctly rounded, x a positive normal number: from the hardware's
 // reciprocal square root (20 bits) two coupled Newton steps for sqrt(x) and
 // 1 / (2 sqrt(x)), then one residual step with the exact remainder (Markstein,

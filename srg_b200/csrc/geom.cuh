@@ -78,25 +78,52 @@ __device__ __forceinline__ void pixel_window(const BurstDev &B, double azoff, in
     }
 }
 
+// x / d correctly rounded, for a divisor whose correctly rounded reciprocal
+// inv is at hand: x inv is within two units in the last place of the quotient,
+// one residual step (exact remainder by FMA, then times inv) makes it faithful
+// and the second one correct (Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000", 1990).  Five operations without a branch, the same
+// bits as the division.
+__device__ __forceinline__ double div_by(double x, double d, double inv) {
+    double q = x * inv;
+    q = fma(fma(-q, d, x), inv, q);
+    return fma(fma(-q, d, x), inv, q);
+}
+
 // 4-point Hermite of position and velocity (sentinel/orbithermite.f:21-70).
+// The reference divides by the differences of the four times throughout; here
+// each difference's reciprocal is taken once (one of a pair, the other is its
+// negative) and the quotients come from div_by, to the same bits: a dependent
+// chain of divisions was most of an azimuth centre's latency.
 __device__ inline void hermite4(const double *x, const double *v, const double *t, double tq,
                                 double *xq, double *vq) {
-    double h[4], hd[4], f0[4], f1[4], g0[4], g1[4];
+    double h[4], hd[4], f0[4], f1[4], g0[4], g1[4], dt[4][4], inv[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < i; ++j) {
+            dt[i][j] = dsub(t[i], t[j]);
+            inv[i][j] = ddiv(1.0, dt[i][j]);
+            dt[j][i] = -dt[i][j];
+            inv[j][i] = -inv[i][j];
+        }
+    double sum[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         f1[i] = dsub(tq, t[i]);
         double s = 0.0;
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            if (j != i) s = dadd(s, ddiv(1.0, dsub(t[i], t[j])));
-        f0[i] = dsub(1.0, dmul(dmul(2.0, dsub(tq, t[i])), s));
+            if (j != i) s = dadd(s, inv[i][j]);
+        sum[i] = s;
+        f0[i] = dsub(1.0, dmul(dmul(2.0, f1[i]), s));
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         double p = 1.0;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            if (k != i) p = ddiv(dmul(p, dsub(tq, t[k])), dsub(t[i], t[k]));
+            if (k != i) p = div_by(dmul(p, f1[k]), dt[i][k], inv[i][k]);
         h[i] = p;
         double s = 0.0;
 #pragma unroll
@@ -104,19 +131,15 @@ __device__ inline void hermite4(const double *x, const double *v, const double *
             double q = 1.0;
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-                if (k != i && k != j) q = ddiv(dmul(q, dsub(tq, t[k])), dsub(t[i], t[k]));
-            if (j != i) s = dadd(s, dmul(ddiv(1.0, dsub(t[i], t[j])), q));
+                if (k != i && k != j) q = div_by(dmul(q, f1[k]), dt[i][k], inv[i][k]);
+            if (j != i) s = dadd(s, dmul(inv[i][j], q));
         }
         hd[i] = s;
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        g1[i] = dadd(h[i], dmul(dmul(2.0, dsub(tq, t[i])), hd[i]));
-        double s = 0.0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (i != j) s = dadd(s, ddiv(1.0, dsub(t[i], t[j])));
-        g0[i] = dmul(2.0, dsub(dmul(f0[i], hd[i]), dmul(h[i], s)));
+        g1[i] = dadd(h[i], dmul(dmul(2.0, f1[i]), hd[i]));
+        g0[i] = dmul(2.0, dsub(dmul(f0[i], hd[i]), dmul(h[i], sum[i])));
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
