@@ -907,9 +907,10 @@ bp_ws(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
                         const float2 *line = B.burst + ((long long)k0 * B.ldb - B.bin0);
                         const long long ldb = B.ldb;
                         const int lo = B.bin0, hi = min(B.bin0 + B.nbins, B.S);
-                        auto pulses = [&](auto proven, int j0, int j1) {
+                        auto pulses = [&](auto proven, auto interior, int j0, int j1) {
                             constexpr bool PROVEN = decltype(proven)::value;
-                            const int wb = h.split ? kWideBins : WB;
+                            constexpr bool INT = decltype(interior)::value;
+                            const int wb = PROVEN || h.split ? kWideBins : WB;
 #pragma unroll 4
                             for (int j = j0; j < j1; ++j) {
                                 const int k = k0 + j;
@@ -923,16 +924,19 @@ bp_ws(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
                                     const float ph = cphp[m] + pa.w;
                                     uacc[m] += dwp;
                                     cphp[m] = fmaf(dwp, Kr, cphp[m]);
-                                    const float fl = floorf(t);
-                                    const int i = (int)fl;
-                                    const float fr = t - fl;
-                                    bool ok = (k >= azs[m]) & (k < aze[m]);
+                                    bool ok = INT || ((k >= azs[m]) & (k < aze[m]));
+                                    float fr;
                                     float2 s0, s1;
-                                    if constexpr (PROVEN) {  // bounded for memory safety
-                                        const int ic = min(max(i, 0), kWideBins - 2);
+                                    if constexpr (PROVEN) {  // floor in the mantissa; bounded for memory safety
+                                        const float tm = __fadd_rd(t, kFloorMagic);
+                                        fr = t - (tm - kFloorMagic);
+                                        const unsigned ic = tap_index<kWideBins>(tm);
                                         s0 = row[ic];
                                         s1 = row[ic + 1];
                                     } else {
+                                        const float fl = floorf(t);
+                                        const int i = (int)fl;
+                                        fr = t - fl;
                                         ok = ok & (t >= h.tlo) & (t <= h.thi);
                                         const bool in = (unsigned)i < (unsigned)(wb - 1);
                                         const int is = in ? i : 0, gi = i + h.x0;
@@ -945,8 +949,10 @@ bp_ws(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
                                     }
                                     float vr = fmaf(fr, s1.x - s0.x, s0.x);
                                     float vi = fmaf(fr, s1.y - s0.y, s0.y);
-                                    vr = ok ? vr : 0.f;
-                                    vi = ok ? vi : 0.f;
+                                    if constexpr (!INT || !PROVEN) {
+                                        vr = ok ? vr : 0.f;
+                                        vi = ok ? vi : 0.f;
+                                    }
                                     float sn, cs;
                                     __sincosf(ph, &sn, &cs);
                                     accr[m] = fmaf(vr, cs, fmaf(-vi, sn, accr[m]));
@@ -958,8 +964,9 @@ bp_ws(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
 #pragma unroll 1
                         for (int j0 = 0;; j0 += kWideRows) {
                             const int j1 = h.split ? min(nk, j0 + kWideRows) : nk;
-                            if (h.split == 2) pulses(std::true_type{}, j0, j1);
-                            else pulses(std::false_type{}, j0, j1);
+                            if (h.split == 2 && h.interior) pulses(std::true_type{}, std::true_type{}, j0, j1);
+                            else if (h.split == 2) pulses(std::true_type{}, std::false_type{}, j0, j1);
+                            else pulses(std::false_type{}, std::false_type{}, j0, j1);
                             if (j1 == nk) break;
                             __syncwarp();
                             if (lane == 0) mbar_arrive(&ctl.empty[s]);
