@@ -765,8 +765,8 @@ int run_bursts(DevCtx &c, const srg_burst_desc *descs, int n, const srg_bp_optio
         const int rc = validate_desc(descs[i]);
         if (rc) return rc;
     }
-    const KernelEntry *ke = gate ? pick_kernel(o.form, o.tile_cfg)
-                                 : pick_default(o.form, o.tile_cfg, descs, n);
+    // (the default's twin has the same tiles, so the drop-in's row blocks hold)
+    const KernelEntry *ke = pick_default(o.form, o.tile_cfg, descs, n);
     if (!ke) return fail(SRG_E_ARG, "no kernel for form %d shape %d", o.form, o.tile_cfg);
     const KernelEntry *twin = gate && n == 1 ? gated_twin(*ke) : nullptr;
     const bool gated = twin != nullptr;

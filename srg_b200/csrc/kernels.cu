@@ -553,7 +553,13 @@ const int kNumKernels = sizeof(kKernels) / sizeof(kKernels[0]);
      (const void *)bp_ws<F, TXv, TYv, NCv, CKv, NSv, WBv, MBv, true>,                           \
      "bp_ws<" #F "," #TXv "x" #TYv ",consumer warps " #NCv ",chunk " #CKv ",stages " #NSv       \
      ",window " #WBv ",min blocks " #MBv ",gated>", 1, 0},
-const KernelEntry kGatedKernels[] = {SRG_WS_GATED_ENTRY(FORM_SPLIT, 32, 8, 4, 31, 2, 128, 3)};
+#define SRG_WIDE_GATED_ENTRY(F, TXv, TYv, NCv, CKv, NSv, WBv, MBv)                              \
+    {F, {TXv, TYv, (NCv + 1) * 32, CKv, WBv}, ws_smem_bytes<F, CKv, NSv>(WBv),                  \
+     (const void *)bp_ws<F, TXv, TYv, NCv, CKv, NSv, WBv, MBv, true, true>,                     \
+     "bp_ws<" #F "," #TXv "x" #TYv ",consumer warps " #NCv ",chunk " #CKv ",stages " #NSv       \
+     ",window " #WBv " or wide,min blocks " #MBv ",gated>", 1, 1},
+const KernelEntry kGatedKernels[] = {SRG_WS_GATED_ENTRY(FORM_SPLIT, 32, 8, 4, 31, 2, 128, 3)
+                                         SRG_WIDE_SHAPES(SRG_WIDE_GATED_ENTRY)};
 const int kNumGatedKernels = sizeof(kGatedKernels) / sizeof(kGatedKernels[0]);
 
 const KernelEntry *gated_twin(const KernelEntry &e) {

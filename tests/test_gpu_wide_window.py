@@ -90,3 +90,23 @@ def test_plan_chooses_again_for_oversampled_lines(orc):
     fine = api.oversample2(db)
     api.backproject([fine], tile_shear=0)
     assert np.array_equal(got, fine.out.cpu().numpy())
+
+
+@pytest.mark.parametrize("spacing,relief,samples", [(2e-4, 0, 2600), (2e-4, 200, 2601), (4e-4, 100, 2600)])
+def test_dropin_on_coarse_grids(spacing, relief, samples):
+    """The drop-in's kernel (lines still arriving) has the same twin: the .geo is
+    the device image, to the bit."""
+    import tempfile
+    b = burst(spacing, relief, samples=samples)
+    db = api.to_device(b)
+    api.backproject([db], tile_cfg=0, tile_shear=0)
+    want = db.out.cpu().numpy()
+    with tempfile.TemporaryFile() as fdem, tempfile.TemporaryFile() as fout:
+        fdem.write(b.dem.tobytes())
+        fdem.flush()
+        fout.truncate(8 * b.demwidth * b.demlength)
+        api.azimuth_compress_status(b, fout.fileno(), fdem.fileno())
+        got = np.memmap(fout, np.complex64, "r", shape=(b.demlength, b.demwidth))
+        rows = np.array(got[db.firstline:db.firstline + db.nlines])
+    merged = np.where(np.abs(want.real) > 1e-18, want, 0)
+    assert np.array_equal(rows, merged)
