@@ -113,11 +113,13 @@ __host__ __device__ constexpr int brev(int i) {
 // rotation that is no quarter turn takes two FMAs for (x + r y, y - r x) with
 // the ratio r of its sine and cosine (at most 1) and four for the sums scaled
 // by the larger of the two: six operations and two roundings per result,
-// against eight and three for the product and its sum and difference.
-template <bool INV>
+// against eight and three for the product and its sum and difference.  The
+// ratio's own rounding shows in long sums, though (range compression's error
+// against 64 bits 2.1e-7, 2.0e-7 without it): FUSED chooses.
+template <bool INV, bool FUSED>
 __device__ __forceinline__ void butterfly(float2 &lo, float2 &hi, int m) {
     const float2 a = lo, b = hi;
-    if (m % 16 == 0) {
+    if (!FUSED || m % 16 == 0) {
         const float2 t = rot64<INV>(b, m);
         hi = csub(a, t);
         lo = cadd(a, t);
@@ -142,7 +144,7 @@ __device__ __forceinline__ void butterfly(float2 &lo, float2 &hi, int m) {
 // R-point DFT (sign -, or + with INV; unnormalised) of v[0..R), in place:
 // input in natural order, bin r of the result in v[brev<R>(r)].  Radix-2
 // decimation in time over the bit-reversed view, so nothing is moved.
-template <int R, bool INV>
+template <int R, bool INV, bool FUSED = true>
 __device__ __forceinline__ void dft(float2 *v) {
 #pragma unroll
     for (int h = 1; h < R; h <<= 1) {
@@ -150,15 +152,16 @@ __device__ __forceinline__ void dft(float2 *v) {
         for (int i = 0; i < R; i += 2 * h) {
 #pragma unroll
             for (int q = 0; q < h; ++q) {
-                butterfly<INV>(v[brev<R>(i + q)], v[brev<R>(i + q + h)], q * (32 / h));
+                butterfly<INV, FUSED>(v[brev<R>(i + q)], v[brev<R>(i + q + h)], q * (32 / h));
             }
         }
     }
 }
 
 // Sizes of one transform and their tables.
-template <int M_, int EPT_, int RA_, int RB_, int RC_>
+template <int M_, int EPT_, int RA_, int RB_, int RC_, bool FUSED_ = true>
 struct Plan {
+    static constexpr bool FUSED = FUSED_;  // butterfly
     static constexpr int M = M_, EPT = EPT_, RA = RA_, RB = RB_, RC = RC_;
     static constexpr int T = M / EPT;            // threads of a line
     static constexpr int CA = M / RA;            // DFTs of pass 1
@@ -266,7 +269,7 @@ __device__ __forceinline__ void conv(float2 (&v)[P::EPT], float2 *buf, int j, in
     // pass 1, from registers
 #pragma unroll
     for (int g = 0; g < P::GA; ++g) {
-        dft<P::RA, false>(v + g * P::RA);
+        dft<P::RA, false, P::FUSED>(v + g * P::RA);
 #pragma unroll
         for (int r = 0; r < P::RA; ++r) {
             const float2 z = v[g * P::RA + brev<P::RA>(r)];
@@ -280,7 +283,7 @@ __device__ __forceinline__ void conv(float2 (&v)[P::EPT], float2 *buf, int j, in
         const int c = j + g * P::T, n2 = c % P::RC;
 #pragma unroll
         for (int r = 0; r < P::RB; ++r) v[r] = buf[P::pass2(c, r)];
-        dft<P::RB, false>(v);
+        dft<P::RB, false, P::FUSED>(v);
 #pragma unroll
         for (int r = 0; r < P::RB; ++r) {
             const float2 z = v[brev<P::RB>(r)];
@@ -296,11 +299,11 @@ __device__ __forceinline__ void conv(float2 (&v)[P::EPT], float2 *buf, int j, in
 #pragma unroll
         for (int g = 0; g < P::GC; ++g) {
             float2 *w = v + g * P::RC;
-            dft<P::RC, false>(w);
+            dft<P::RC, false, P::FUSED>(w);
             float2 u[P::RC];
 #pragma unroll
             for (int r = 0; r < P::RC; ++r) u[r] = mul(w[brev<P::RC>(r)], g * P::RC + r, j);
-            dft<P::RC, true>(u);
+            dft<P::RC, true, P::FUSED>(u);
 #pragma unroll
             for (int r = 0; r < P::RC; ++r) row[g * P::RC + r] = u[brev<P::RC>(r)];
         }
@@ -315,7 +318,7 @@ __device__ __forceinline__ void conv(float2 (&v)[P::EPT], float2 *buf, int j, in
             const float2 z = buf[P::pass2(c, r)];
             v[r] = r ? cmulc(z, iw2[(r - 1) * P::RC + n2]) : z;
         }
-        dft<P::RB, true>(v);
+        dft<P::RB, true, P::FUSED>(v);
 #pragma unroll
         for (int r = 0; r < P::RB; ++r) buf[P::pass2(c, r)] = v[brev<P::RB>(r)];
     }
@@ -329,7 +332,7 @@ __device__ __forceinline__ void conv(float2 (&v)[P::EPT], float2 *buf, int j, in
             const float2 z = buf[P::pad_from(pj, j, g * P::T + r * P::CA)];
             u[r] = r ? cmulc(z, iw1(r, j, g)) : z;
         }
-        dft<P::RA, true>(u);
+        dft<P::RA, true, P::FUSED>(u);
 #pragma unroll
         for (int r = 0; r < P::RA; ++r) v[g * P::RA + r] = u[brev<P::RA>(r)];
     }

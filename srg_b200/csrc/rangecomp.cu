@@ -90,14 +90,16 @@ __global__ void rc_out_kernel(const float2 *__restrict__ buf, int l0, int nlines
 // memory (fft_conv.cuh) with the filter H = (32768 / 8192) conj(DFT_8192(r))
 // and writes its L outputs once: the lines cross HBM once each way, where the
 // cuFFT path below takes five passes over 32,768-point rows.  A CTA takes two
-// segments at once, 256 threads each, that share the filter's spectrum (64 KB)
-// and pass 1's twiddles (30 KB) in shared memory.  Bound by instruction issue
-// (see fft_conv.cuh): 1,500 lines of 24,000 samples, pulse of 3,371, take
-// 0.30 ms (0.45 with self-sorting transforms of one segment per 512-thread CTA),
-// 700 lines of 29,001 with a pulse of 5,147 0.23 ms (0.58 with cuFFT).  The same
-// with the tables read through L1 and two CTAs per SM: 0.31 ms; as two halves
-// of 4,096 points at 16 points per thread: 0.42 ms.
-using Seg = fftc::Plan<8192, 32, 16, 16, 32>;
+// segments at once, 256 threads each, that share the twiddles (62 KB) in shared
+// memory; the filter's spectrum (64 KB, once per segment) is read through L1.
+// Bound by instruction issue (see fft_conv.cuh): 1,500 lines of 24,000 samples,
+// pulse of 3,371, take 0.31 ms (0.45 with self-sorting transforms of one segment
+// per 512-thread CTA), 700 lines of 29,001 with a pulse of 5,147 0.24 ms (0.58
+// with cuFFT).  With fused butterflies (Plan::FUSED) 0.29 ms and 5 % more error;
+// with the spectrum in shared memory and half the twiddles turned from the
+// others 0.30 and 10 % more; everything through L1 and two CTAs per SM 0.31, as two
+// halves of 4,096 points at 16 points per thread 0.42.
+using Seg = fftc::Plan<8192, 32, 16, 16, 32, false>;
 constexpr int kOsM = Seg::M;                     // segment transform
 // Segments per line up to which the kernel is the faster path: one takes
 // 41 ns (of the whole chip), a line of the cuFFT path 0.84 us whatever its
@@ -105,7 +107,17 @@ constexpr int kOsM = Seg::M;                     // segment transform
 constexpr int kOsMaxSegs = 20;
 constexpr int kOsLines = 2;                      // segments of a CTA at once
 constexpr int kOsThreads = kOsLines * Seg::T;
-constexpr int kOsSmem = (kOsLines * Seg::BUF + kOsM + Seg::TW1) * (int)sizeof(float2);
+// pass 1's twiddles of every column in shared memory (exactly rounded: turned
+// from the first columns' they cost 5 % more error); pass 2's are read through
+// L1 (in shared memory as well they leave L1 too small for the spectrum: 0.33 ms)
+constexpr int kOsTw1 = (Seg::RA - 1) * Seg::CA;
+constexpr int kOsSmem = (kOsLines * Seg::BUF + kOsTw1) * (int)sizeof(float2);
+struct SegTw1 {
+    const float2 *t;
+    __device__ __forceinline__ float2 operator()(int r, int j, int g) const {
+        return t[(r - 1) * Seg::CA + j + g * Seg::T];
+    }
+};
 
 __global__ void __launch_bounds__(kOsThreads, 1)
 rc_os_kernel(const float2 *__restrict__ in, long long ld_in, int nsamps, int nvalid, int L,
@@ -114,12 +126,12 @@ rc_os_kernel(const float2 *__restrict__ in, long long ld_in, int nsamps, int nva
     extern __shared__ float2 os_sm[];
     const int j = threadIdx.x % Seg::T, slot = threadIdx.x / Seg::T;
     float2 *buf = os_sm + slot * Seg::BUF;
-    float2 *h = os_sm + kOsLines * Seg::BUF, *t1 = h + kOsM;
-    for (int i = threadIdx.x; i < kOsM; i += kOsThreads) h[i] = __ldg(H + i);
-    for (int i = threadIdx.x; i < Seg::TW1; i += kOsThreads) t1[i] = __ldg(tw + i);
+    float2 *t1 = os_sm + kOsLines * Seg::BUF;
+    for (int i = threadIdx.x; i < kOsTw1; i += kOsThreads) t1[i] = __ldg(tw + i);
     __syncthreads();
-    const fftc::Tw1<Seg> tw1{t1};
-    const fftc::Filter<Seg> filter{h};
+    const SegTw1 tw1{t1};
+    const float2 *tw2 = tw + kOsTw1;
+    const fftc::Filter<Seg> filter{H};
     const int step = gridDim.x * kOsLines;
     for (int item = blockIdx.x * kOsLines + slot; item < nitems; item += step) {
         const int line = item / nseg, s0 = (item - line * nseg) * L;
@@ -137,7 +149,7 @@ rc_os_kernel(const float2 *__restrict__ in, long long ld_in, int nsamps, int nva
             for (int c = 16 * j; c < min(kOsM, nsamps - ns); c += 16 * Seg::T)
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + c));
         }
-        fftc::conv<Seg>(v, buf, j, slot, false, tw1, tw + Seg::TW1, tw1, tw + Seg::TW1, filter);
+        fftc::conv<Seg>(v, buf, j, slot, false, tw1, tw2, tw1, tw2, filter);
         float2 *y = out + (long long)line * ld_out + s0 + j;
         const int nout = min(L, nvalid - s0) - j;
 #pragma unroll
@@ -242,10 +254,18 @@ int srg_range_compress_device(const float *lines, long long ld_in, int nlines, i
     if (nseg > 0 && nseg <= kOsMaxSegs) {
         // fused overlap-save kernel (see rc_os_kernel)
         if ((rc = x.os_h.ensure(sizeof(float2) * kOsM)) ||
-            (rc = x.os_tw.ensure(sizeof(float2) * (Seg::TW1 + Seg::TW2))))
+            (rc = x.os_tw.ensure(sizeof(float2) * (kOsTw1 + Seg::TW2))))
             return rc;
         if (!x.os_ready) {
-            const std::vector<float2> tw = fftc::tables<Seg>(0.0);
+            std::vector<float2> tw;
+            const std::vector<float2> plan = fftc::tables<Seg>(0.0);
+            const double tau = 8.0 * std::atan2(1.0, 1.0);
+            for (int r = 1; r < Seg::RA; ++r)
+                for (int d = 0; d < Seg::CA; ++d) {
+                    const double a = tau * r * d / Seg::M;
+                    tw.push_back(make_float2((float)std::cos(a), (float)-std::sin(a)));
+                }
+            tw.insert(tw.end(), plan.begin() + Seg::TW1, plan.end());
             int sms = 0;
             CKR(cudaFuncSetAttribute(rc_os_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kOsSmem));
             CKR(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
