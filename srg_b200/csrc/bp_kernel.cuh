@@ -195,6 +195,13 @@ __device__ __forceinline__ void sincos_pos(double x, double *sn, double *cs) {
     *cs = __hiloint2double(__double2hiint(b) ^ (((q + 1) << 30) & 0x80000000), __double2loint(b));
 }
 
+// A satellite coordinate as the terms of bp_tiles take it.  The loop evaluates a
+// term that does not count beside one that does and multiplies its sine and
+// cosine by a zero sample, so they must be numbers: a coordinate that is none, or
+// whose range would overflow, becomes one far out of every range (its phase's
+// polynomials stay below 1e240).
+__device__ __forceinline__ double term_position(double s) { return fabs(s) < 1e30 ? s : 1e30; }
+
 // Stages pulses [k0, k0 + rows) x bins [x0, x0 + wb) of a burst without a TMA
 // descriptor (odd row strides, unaligned lines) by asynchronous copies of
 // single samples, thread t of n: every copy is in flight at once, where
@@ -432,10 +439,13 @@ bp_tiles(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
                         p[2] = make_float4(__double2float_rn(0.5 * iR), __double2float_rn(iR), 0.f, 0.f);
                     } else {
                         double *p = prmd + 4 * lane;
-                        p[0] = sx;
-                        p[1] = sy;
-                        p[2] = sz;
+                        p[0] = term_position(sx);
+                        p[1] = term_position(sy);
+                        p[2] = term_position(sz);
                     }
+                } else if (FORM == FORM_FP64 && lane < CK) {
+                    double *p = prmd + 4 * lane;  // read beside an odd chunk's last pulse
+                    p[0] = p[1] = p[2] = 0.0;
                 }
                 int lo = on ? (int)floor(rbabs) : INT_MAX;
                 int hi = on ? (int)ceil(rbabs) : INT_MIN;
@@ -536,7 +546,7 @@ bp_tiles(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
                         bool ok[E], any = false;
 #pragma unroll
                         for (int e = 0; e < E; ++e) {
-                            // (pulse nk of an odd chunk: whatever the stage holds there, not ok)
+                            // (pulse nk of an odd chunk: a row of zeros, not ok)
                             const int m = e % M, jj = j + e / M;
                             const double vx = dsub(X[m][0], prmd[4 * jj + 0]),
                                          vy = dsub(X[m][1], prmd[4 * jj + 1]),
