@@ -278,6 +278,14 @@ std::vector<float2> plan_tables() {
     return all;
 }
 
+// What the odd samples are to be multiplied by for the transforms' gain
+// (fft_conv.cuh), to the 1.2e-7 of a factor next to 1; C > 1: odd_cluster_kernel's.
+template <class P, int C = 1>
+__host__ __device__ constexpr float odd_correction() {
+    constexpr double gain = fftc::conv_gain<P>() + fftc::half_sample_gain<P>() + fftc::dft_gain<C>();
+    return (float)(1.0 / (1.0 + gain));
+}
+
 // The odd upsampled samples (unnormalised) of the line in v.
 template <class P>
 __device__ __forceinline__ void odd_samples(float2 (&v)[P::EPT], float2 *buf, int j, int slot,
@@ -492,7 +500,7 @@ odd_stack_kernel(const __grid_constant__ StackPtrs p, int n, long long ld, int n
     for (int i = threadIdx.x; i < 2 * table_entries<P>(); i += NT) tab[i] = __ldg(tabg + i);
     __syncthreads();
     // results / nnn / 2: powers of two, applied to the input for the odd samples
-    const float odd_scale = scale * (0.5f / (float)P::M), even_scale = scale * 0.5f;
+    const float odd_scale = scale * (0.5f / (float)P::M * odd_correction<P>()), even_scale = scale * 0.5f;
     const long long steps = (long long)nlines * n;
     const int w = blockIdx.x * LP + slot;
     const long long s0 = w < workers ? steps * w / workers : 0;
@@ -643,6 +651,7 @@ struct OwnPlan {
     const void *stack;  // odd_stack_kernel for single looks, or null
     const void *across; // the same for looks of several columns, one line down
     int threads, lines, smem, cluster;
+    float correction;   // odd_correction
     std::vector<float2> (*tables)();
 };
 template <int C>
@@ -661,12 +670,12 @@ template <class P>
 OwnPlan small_plan() {
     return {P::M, (const void *)odd_kernel<P>, (const void *)odd_stack_kernel<P, false>,
             (const void *)odd_stack_kernel<P, true>, cta_threads<P>(),
-            lines_per_cta<P>(), odd_smem<P>(), 1, plan_tables<P>};
+            lines_per_cta<P>(), odd_smem<P>(), 1, odd_correction<P>(), plan_tables<P>};
 }
 template <int C>
 OwnPlan cluster_plan() {
     return {C * P8192::M, (const void *)odd_cluster_kernel<C>, nullptr, nullptr, P8192::T, 1,
-            (int)sizeof(float2) * (P8192::BUF + P8192::EPT), C, cluster_tables<C>};
+            (int)sizeof(float2) * (P8192::BUF + P8192::EPT), C, odd_correction<P8192, C>(), cluster_tables<C>};
 }
 constexpr int kOwnPlans = 11;
 const OwnPlan *own_plans() {
@@ -674,7 +683,7 @@ const OwnPlan *own_plans() {
         small_plan<P64>(), small_plan<P128>(), small_plan<P256>(), small_plan<P512>(),
         small_plan<P1024>(), small_plan<P2048>(), small_plan<P4096>(),
         {P8192::M, (const void *)odd_kernel<P8192>, nullptr, nullptr, P8192::T, 1, odd_smem<P8192>(), 1,
-         plan_tables<P8192>},
+         odd_correction<P8192>(), plan_tables<P8192>},
         cluster_plan<2>(), cluster_plan<4>(), cluster_plan<8>()};
     return plans;
 }
@@ -860,7 +869,7 @@ int run_stack(const float *const *slcs, int n, long long ld, int na, int nlines,
     const long long ldo = own >= 0 ? na : 2LL * nnn;
     // the reference's divisions (by a power of two), and the input's scale where
     // the odd samples do not have it yet
-    const float of = 0.5f / (float)nnn * (own >= 0 ? scale : 1.f);
+    const float of = 0.5f / (float)nnn * (own >= 0 ? scale * own_plans()[own].correction : 1.f);
     for (int k = 0; k + 1 < n; ++k) {
         const float2 *a = reinterpret_cast<const float2 *>(slcs[k]);
         const float2 *b = reinterpret_cast<const float2 *>(slcs[k + 1]);
