@@ -278,8 +278,9 @@ int srg_range_compress_device(const float *lines, long long ld_in, int nlines, i
         }
         const float key[4] = {samplefreq, startfreq, ramprate, pulselength};
         if (std::memcmp(key, x.os_key, sizeof key) != 0) {
-            // H = (32768 / 8192) conj(DFT_8192(replica)), in FP64 from the
-            // replica's complex64 samples
+            // H = (32768 / 8192) conj(DFT_8192(replica)), less the transforms' gain
+            // (they return 1.0e-7 too little, half of the error against 64 bits), in
+            // FP64 from the replica's complex64 samples
             std::vector<float> rep(2 * (size_t)kOsM);
             if ((rc = srg_range_replica(samplefreq, startfreq, ramprate, pulselength, rep.data(), kOsM,
                                         &npts)))
@@ -288,7 +289,7 @@ int srg_range_compress_device(const float *lines, long long ld_in, int nlines, i
             for (int j = 0; j < npts; ++j) a[j] = std::complex<double>(rep[2 * j], rep[2 * j + 1]);
             host_fft(a);
             std::vector<float2> h(kOsM);
-            const double scale = (double)kRangeFFT / kOsM;
+            const double scale = (double)kRangeFFT / kOsM / (1.0 + fftc::conv_gain<Seg>());
             for (int i = 0; i < Seg::EPT; ++i)
                 for (int j = 0; j < Seg::T; ++j) {
                     const std::complex<double> b = a[fftc::spectrum_order<Seg>(i, j)];
