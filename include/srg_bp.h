@@ -302,7 +302,8 @@ int srg_scene_tune(srg_scene *s, int iters, int *best_cfg, double *best_ms);
  * the kernel shapes of the plan's form, unless use_cache finds the best shape
  * of an earlier tuning of a scene of the same shape (same form,
  * interpolation, and bursts' pulses, samples, grid lines and columns to
- * within 64, 1024, 64, 64); results are kept for the process and, when the
+ * within 64, 1024, 64, 64; bursts on coarse grids or without a TMA descriptor
+ * only match such bursts); results are kept for the process and, when the
  * environment variable SRG_TUNE_CACHE names a file, appended to it and read
  * back by later processes.  srg_scene_tune is this with no interpolation
  * budget and the cache on.  No reference counterpart. */

@@ -359,7 +359,7 @@ StreamValueOps stream_value_ops() {
 }
 
 // The lines' base and row stride suit a TMA descriptor (16-byte units).
-static bool tma_lines(const BurstDev &B) {
+bool tma_lines(const BurstDev &B) {
     return !(reinterpret_cast<uintptr_t>(B.burst) & 15) && !((B.ldb * 8) & 15) && !(B.bin0 & 1);
 }
 
@@ -374,6 +374,10 @@ const KernelEntry *pick_kernel(int form, int cfg) {
     return nullptr;
 }
 
+double tile_bins(const BurstDev &B, const KernelEntry &ke) {
+    return std::fabs(B.rbin_col) * (ke.shape.tx - 1) + std::fabs(B.rbin_line) * (ke.shape.ty - 1) + 8.0;
+}
+
 // The default shape of a launch over n bursts (KernelEntry order decides
 // elsewhere).  The split form's first shape stages 128 range bins; a 32 x 8
 // tile's pixels spread over |bins per column| 31 + |bins per line| 7 of them on
@@ -382,17 +386,14 @@ const KernelEntry *pick_kernel(int form, int cfg) {
 // column: coarse pixels, oversampled lines) get the twin of that shape with
 // wide stages, whose results are the same; so do lines that have no TMA
 // descriptor (odd row strides), which the twin stages asynchronously (1,500
-// pulses of 21,001 samples: 1.3 ms, 7.7 in the first shape).  kFlat leaves room
-// for the relief inside a tile; below it the twin costs up to 1 %.
+// pulses of 21,001 samples: 1.3 ms, 7.7 in the first shape).  kFlatBins leaves
+// room for the relief inside a tile; below it the twin costs up to 1 %.
 const KernelEntry *pick_default(int form, int cfg, const srg_burst_desc *descs, int n) {
     const KernelEntry *ke = pick_kernel(form, cfg);
     if (!ke || cfg >= 0 || form != SRG_FORM_SPLIT) return ke;
-    constexpr double kFlat = 112.0;
     for (int i = 0; i < n; ++i) {
         const BurstDev B = make_burst_dev(descs[i], nullptr);
-        const double need = std::fabs(B.rbin_col) * (ke->shape.tx - 1) +
-                            std::fabs(B.rbin_line) * (ke->shape.ty - 1) + 8.0;
-        if (!(need > kFlat) && tma_lines(B)) continue;
+        if (!(tile_bins(B, *ke) > kFlatBins) && tma_lines(B)) continue;
         for (int k = 0; k < kNumKernels; ++k)
             if (kKernels[k].form == form && kKernels[k].wide) return &kKernels[k];
     }

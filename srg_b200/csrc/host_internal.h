@@ -109,6 +109,12 @@ struct StreamValueOps {
 StreamValueOps stream_value_ops();
 // Streams, events and pinned error word of the drop-in entry (made once).
 int ensure_dropin(DevCtx &c);
+// The lines' base and row stride suit a TMA descriptor.
+bool tma_lines(const BurstDev &B);
+// Range bins that a tile of `ke` spreads over on flat earth and that its window
+// needs for margins; above kFlatBins pick_default takes the wide twin.
+double tile_bins(const BurstDev &B, const KernelEntry &ke);
+constexpr double kFlatBins = 112.0;
 // Kernel entry for a form and shape index (-1: the default of that form).
 const KernelEntry *pick_kernel(int form, int cfg);
 // The same for a launch over the given (valid) bursts: the default takes their

@@ -264,15 +264,24 @@ const char *tune_file() {
 }
 
 // Scene shape: the multiset of (pulses / 64, samples / 1024, lines / 64,
-// columns / 64) of its bursts, with the form and the interpolation.
+// columns / 64) of its bursts, with the form and the interpolation.  Bursts
+// for which the default shape is not the first one, by the same measures, say
+// why: /b and the bins of a tile / 64 where its window does not hold them,
+// /u where the lines have no TMA descriptor.  (A shape that was the fastest on
+// a fine grid can be six times slower there.  Keys of other bursts are those of
+// files written without these marks.)
 std::string tune_key(const srg_scene *s) {
     std::vector<std::string> parts;
+    const KernelEntry &ke = *pick_kernel(s->opts.form, -1);
     for (int i = 0; i < s->n; ++i) {
         const BurstDev &B = s->hb[i];
         char buf[96];
         snprintf(buf, sizeof buf, "%d/%d/%d/%d", B.P / 64, B.S / 1024, B.nlines / 64,
                  (B.lastpix_eff - B.firstpix + 1) / 64);
         parts.emplace_back(buf);
+        const double bins = tile_bins(B, ke);
+        if (bins > kFlatBins) parts.back() += "/b" + std::to_string((int)std::min(bins / 64.0, 1e6));
+        if (!tma_lines(B)) parts.back() += "/u";
     }
     std::sort(parts.begin(), parts.end());
     std::string k = "f" + std::to_string(s->opts.form) + ":i" + std::to_string(s->interp) + ":";
