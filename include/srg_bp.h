@@ -420,6 +420,12 @@ int srg_bp_burst_device_noalloc(const srg_burst_desc *b, const srg_bp_options *o
  * sets it near there to run calls across the restart. */
 int srg_test_set_dropin_sequence(int device, int seq);
 
+/* Testing hook: the FP64 form's own steps of a term, as device code, on n (at
+ * least 1) values: root[i] = sqrt(x[i]), quot[i] = x[i] / d[i], sn[i] and cs[i]
+ * the sine and cosine of x[i].  Device pointers; enqueued on `stream`. */
+int srg_test_fp64_steps_device(const double *x, const double *d, int64_t n, double *root,
+                               double *quot, double *sn, double *cs, void *stream);
+
 /* Calibration: measured FMA issue-rate peak of the current device in
  * TFLOP/s (2 flops per FMA), FP32 (fp64 = 0) or FP64 (fp64 = 1), from a
  * full-occupancy chain-of-FMA kernel timed with CUDA events.  Blocking. */

@@ -144,7 +144,7 @@ __device__ __forceinline__ float2 ld_where(bool use, const float2 *p, float2 v) 
 }
 
 // ---- FP64 steps of a term ----
-// sqrt(x) correctly rounded, x a positive normal number: from the hardware's
+// sqrt(x) correctly rounded, x from 2^-900 to 2^1000: from the hardware's
 // reciprocal square root (20 bits) two coupled Newton steps for sqrt(x) and
 // 1 / (2 sqrt(x)), then one residual step with the exact remainder (Markstein,
 // "IA-64 and elementary functions", 2000).  Eleven operations and no branch, the
@@ -162,12 +162,12 @@ __device__ __forceinline__ double sqrt_pos(double x) {
     return fma(fma(-g, g, x), h, g);
 }
 
-// sin and cos of x, 0 <= x < 2^30, within one unit in the last place: x less
+// sin and cos of x, 0 <= x < 2^30, to 1.2 * 2^-53 (absolute): x less
 // the nearest multiple n of pi/2 in two parts (Cody and Waite; the first
 // product and difference are exact in an FMA: x has no bits below 2^-23 that
 // pi/2's do not reach, and the remainder is below 1), then polynomials through
 // the Chebyshev points of the interval (interpolated in rational arithmetic;
-// errors 1.8e-17 and 9e-19).  24 FP64 operations and no branch.
+// errors 1.8e-17 and 9e-19).  19 FP64 operations and no branch.
 constexpr double kSinCosMax = 1073741824.0;
 __device__ __forceinline__ void sincos_pos(double x, double *sn, double *cs) {
     const double magic = 6755399441055744.0;  // 1.5 * 2^52: rounds to an integer in the low word

@@ -1133,6 +1133,14 @@ int srg_forward_project_device(const srg_burst_desc *b, const float *refl, int64
     return SRG_OK;
 }
 
+int srg_test_fp64_steps_device(const double *x, const double *d, int64_t n, double *root,
+                               double *quot, double *sn, double *cs, void *stream) {
+    if (!x || !d || !root || !quot || !sn || !cs || n < 1 || n > (1LL << 31))
+        return fail(SRG_E_ARG, "bad arguments");
+    CK(launch_fp64_steps(x, d, n, root, quot, sn, cs, static_cast<cudaStream_t>(stream)));
+    return SRG_OK;
+}
+
 int srg_measure_fma_peak(int fp64, double *tflops) {
     if (!tflops) return fail(SRG_E_ARG, "null output");
     DevCtx *c = nullptr;

@@ -83,7 +83,9 @@ __device__ __forceinline__ void pixel_window(const BurstDev &B, double azoff, in
 // one residual step (exact remainder by FMA, then times inv) makes it faithful
 // and the second one correct (Markstein, "Computation of elementary functions on
 // the IBM RISC System/6000", 1990).  Five operations without a branch, the same
-// bits as the division.
+// bits as the division for |x| above 2^-900, say, where no remainder is lost
+// below the normal numbers, and for zeros, but that -0 / d of a positive d
+// comes out as +0 (div_by(-x, -d, -inv) keeps its sign).
 __device__ __forceinline__ double div_by(double x, double d, double inv) {
     double q = x * inv;
     q = fma(fma(-q, d, x), inv, q);
@@ -94,7 +96,9 @@ __device__ __forceinline__ double div_by(double x, double d, double inv) {
 // The reference divides by the differences of the four times throughout; here
 // each difference's reciprocal is taken once (one of a pair, the other is its
 // negative) and the quotients come from div_by, to the same bits: a dependent
-// chain of divisions was most of an azimuth centre's latency.
+// chain of divisions was most of an azimuth centre's latency.  (A zero quotient,
+// at one of the four times, is only ever added to or multiplied, so the sign that
+// div_by may lose changes no other number; keeping it cost 1.6 us of 14.5.)
 __device__ inline void hermite4(const double *x, const double *v, const double *t, double tq,
                                 double *xq, double *vq) {
     double h[4], hd[4], f0[4], f1[4], g0[4], g1[4], dt[4][4], inv[4][4];

@@ -494,6 +494,24 @@ cudaError_t launch_fma_peak(int fp64, int blocks, int iters, void *sink, cudaStr
     return cudaGetLastError();
 }
 
+__global__ void __launch_bounds__(256)
+fp64_steps_kernel(const double *__restrict__ x, const double *__restrict__ d, long long n,
+                  double *__restrict__ root, double *__restrict__ quot, double *__restrict__ sn,
+                  double *__restrict__ cs) {
+    const long long i = blockIdx.x * 256LL + threadIdx.x;
+    if (i >= n) return;
+    root[i] = sqrt_pos(x[i]);
+    const double inv = ddiv(1.0, d[i]);
+    quot[i] = signbit(x[i]) && d[i] > 0.0 ? div_by(-x[i], -d[i], -inv) : div_by(x[i], d[i], inv);
+    sincos_pos(x[i], sn + i, cs + i);
+}
+
+cudaError_t launch_fp64_steps(const double *x, const double *d, long long n, double *root,
+                              double *quot, double *sn, double *cs, cudaStream_t st) {
+    fp64_steps_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(x, d, n, root, quot, sn, cs);
+    return cudaGetLastError();
+}
+
 // ---------------------------------------------------------------------------
 // Compiled shapes.  First generation (bp_tiles): {form, tile_x, tile_y,
 // threads, chunk, window}.  Warp-specialised (bp_ws): {form, tile_x, tile_y,

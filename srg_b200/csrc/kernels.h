@@ -88,6 +88,8 @@ cudaError_t launch_forward_project(const BurstDev &B, const float2 *refl, long l
                                    const double *satvel, double antenna, const float *range_offset,
                                    cudaStream_t st);
 
+cudaError_t launch_fp64_steps(const double *x, const double *d, long long n, double *root,
+                              double *quot, double *sn, double *cs, cudaStream_t st);
 cudaError_t launch_fma_peak(int fp64, int blocks, int iters, void *sink, cudaStream_t st);
 
 inline int shared_bytes(const KernelEntry &e) { return e.smem; }
