@@ -470,7 +470,7 @@ int srg_forward_project_device(const srg_burst_desc *b, const float *refl,
  * with cuFFT the upsampled images) is shared by every call on it: calls on
  * the same device whose GPU work overlaps (other streams) race, except those
  * that form the pairs without scratch: looks of one line down (looksdn = 1)
- * of lines of 33-4,096 samples.
+ * of lines of 33-4,096 samples, scale 0 or at least 1e-30 in magnitude.
  */
 int srg_crossmul_device(const float *slc1, const float *slc2, long long ld, int na, int nlines,
                         int looksac, int looksdn, float scale, int mask, float *igram,

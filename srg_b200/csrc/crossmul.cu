@@ -307,8 +307,10 @@ __device__ __forceinline__ void load_line(float2 (&v)[P::EPT], const float2 *__r
     }
 }
 
-// Odd samples of every line of one or two images, not yet scaled, into odd[0],
-// odd[1] ([nl][na]).  Launch and latency bound at small sizes: a 917 x 601 pair
+// Odd samples of every line of one or two images, of in * scale (multiplied
+// first, as the reference does: a scale may bring samples into range that the
+// sums of a line would leave) and not yet / nnn / 2, into odd[0], odd[1]
+// ([nl][na]).  Launch and latency bound at small sizes: a 917 x 601 pair
 // with looks takes 19 us in two launches (72 us in seven with cuFFT).  Persistent, kThreads / T lines of a CTA at once.
 struct OddArgs {
     const float2 *in[2];
@@ -316,7 +318,7 @@ struct OddArgs {
 };
 template <class P>
 __global__ void __launch_bounds__(cta_threads<P>(), 2)
-odd_kernel(const __grid_constant__ OddArgs a, int nimg, long long ld, int na, int nl,
+odd_kernel(const __grid_constant__ OddArgs a, int nimg, long long ld, int na, int nl, float scale,
            const float2 *__restrict__ tabg) {
     extern __shared__ float2 xm_sm[];
     constexpr int LP = lines_per_cta<P>();
@@ -337,6 +339,8 @@ odd_kernel(const __grid_constant__ OddArgs a, int nimg, long long ld, int na, in
         const long long l = mine ? item - (long long)k * nl : 0;
         float2 v[P::EPT];
         load_line<P, !tables_in_smem<P>()>(v, a.in[k] + l * ld, j, mine ? na : 0);
+#pragma unroll
+        for (int i = 0; i < P::EPT; ++i) v[i] = make_float2(v[i].x * scale, v[i].y * scale);
         odd_samples<P>(v, buf, j, slot, LP == 1, tab);
         float2 *out = a.odd[k] + l * na + j;
         const int nm = mine ? na - j : 0;
@@ -378,7 +382,7 @@ __device__ __forceinline__ float2 ld_cluster(unsigned addr) {
 template <int C>
 __global__ void __launch_bounds__(P8192::T, 2)
 odd_cluster_kernel(const __grid_constant__ OddArgs a, int nimg, long long ld, int na, int nl,
-                   const float2 *__restrict__ tabg) {
+                   float scale, const float2 *__restrict__ tabg) {
     using P = P8192;
     namespace cg = cooperative_groups;
     extern __shared__ float2 xm_sm[];
@@ -403,6 +407,8 @@ odd_cluster_kernel(const __grid_constant__ OddArgs a, int nimg, long long ld, in
         const float2 *x = a.in[k] + l * ld;
         float2 v[P::EPT];
         load_line<P, true>(v, x, j, na);
+#pragma unroll
+        for (int i = 0; i < P::EPT; ++i) v[i] = make_float2(v[i].x * scale, v[i].y * scale);
         if (item + gridDim.x / C < items) {  // this CTA's share of the next line into L2
             const long long ni = item + gridDim.x / C;
             const float2 *nx = ni >= nl ? a.in[1] + (ni - nl) * ld : a.in[0] + ni * ld;
@@ -412,7 +418,9 @@ odd_cluster_kernel(const __grid_constant__ OddArgs a, int nimg, long long ld, in
 #pragma unroll 1
         for (int c = 1; c < C; ++c) {
             if (c * P::M >= na) break;
-            const float2 wc = __ldg(root + (q * c * P::EPT) % (P::EPT * C));  // exp(-2 pi i q c / C)
+            // scale exp(-2 pi i q c / C)
+            const float2 w1 = __ldg(root + (q * c * P::EPT) % (P::EPT * C));
+            const float2 wc = make_float2(w1.x * scale, w1.y * scale);
 #pragma unroll
             for (int m0 = 0; m0 < P::EPT; m0 += 16) {  // in the order of the line
                 if (m0 * P::T + c * P::M >= na) break;
@@ -766,11 +774,12 @@ int ensure_plan(XmCtx &x, int i, int dev, cudaStream_t st) {
 }
 
 // odd samples of nimg (1 or 2) images by own plan `i`
-int launch_odd(XmCtx &x, int i, OddArgs a, int nimg, long long ld, int na, int nl, cudaStream_t st) {
+int launch_odd(XmCtx &x, int i, OddArgs a, int nimg, long long ld, int na, int nl, float scale,
+               cudaStream_t st) {
     const OwnPlan &p = own_plans()[i];
     const long long groups = ((long long)nimg * nl + p.lines - 1) / p.lines;
     const float2 *tab = static_cast<const float2 *>(x.tab[i].p);
-    void *args[] = {&a, &nimg, &ld, &na, &nl, (void *)&tab};
+    void *args[] = {&a, &nimg, &ld, &na, &nl, &scale, (void *)&tab};
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute at{};
     cluster_config(p, (int)std::min<long long>(groups * p.cluster, x.odd_ctas[i]), st, cfg, at);
@@ -834,7 +843,9 @@ int run_stack(const float *const *slcs, int n, long long ld, int na, int nlines,
     if (own >= 0) {
         if ((rc = ensure_plan(x, own, dev, st))) return rc;
         const OwnPlan &op = own_plans()[own];
-        if (op.stack && looksdn == 1) {
+        // (odd_stack_kernel takes scale / nnn / 2 as one factor, which must be a
+        // normal number)
+        if (op.stack && looksdn == 1 && (std::fabs(scale) >= 1e-30f || scale == 0.f)) {
             const void *fn = looksac == 1 ? op.stack : op.across;
             const int ctas = (looksac == 1 ? x.stack_ctas : x.across_ctas)[own];
             const float2 *tab = static_cast<const float2 *>(x.tab[own].p);
@@ -867,9 +878,8 @@ int run_stack(const float *const *slcs, int n, long long ld, int na, int nlines,
     float2 *cur = static_cast<float2 *>(x.upA.p), *nxt = static_cast<float2 *>(x.upB.p);
     const int off = own >= 0 ? 0 : 1, os = own >= 0 ? 1 : 2;
     const long long ldo = own >= 0 ? na : 2LL * nnn;
-    // the reference's divisions (by a power of two), and the input's scale where
-    // the odd samples do not have it yet
-    const float of = 0.5f / (float)nnn * (own >= 0 ? scale * own_plans()[own].correction : 1.f);
+    // the reference's divisions (by a power of two)
+    const float of = 0.5f / (float)nnn * (own >= 0 ? own_plans()[own].correction : 1.f);
     for (int k = 0; k + 1 < n; ++k) {
         const float2 *a = reinterpret_cast<const float2 *>(slcs[k]);
         const float2 *b = reinterpret_cast<const float2 *>(slcs[k + 1]);
@@ -885,7 +895,7 @@ int run_stack(const float *const *slcs, int n, long long ld, int na, int nlines,
                 oa.in[m] = b;
                 oa.odd[m++] = nxt;
             }
-            if (m && (rc = launch_odd(x, own, oa, m, ld, na, nl, st))) return rc;
+            if (m && (rc = launch_odd(x, own, oa, m, ld, na, nl, scale, st))) return rc;
         } else {
             if (k == 0 && (rc = upsample(x, a, ld, na, nnn, nl, scale, cur, st))) return rc;
             if (!same && (rc = upsample(x, b, ld, na, nnn, nl, scale, nxt, st))) return rc;
