@@ -669,10 +669,13 @@ bp_ws(const BurstDev *__restrict__ bursts, int nbursts, int total_tiles,
                     gave_up = true;
                     break;
                 }
-                // Range lines still in transfer: wait (bounded) until the rows
-                // of this chunk are in device memory.
+                // Range lines still in transfer: wait (bounded) until every row that
+                // this chunk's copies read is in device memory (a wide chunk's two
+                // stages read 32, one more than it has pulses).
                 if (GATE && ready) {
-                    const int target = ready_base + (min(k0 + CK, Pm1 + 1) + ready_rows - 1) / ready_rows;
+                    constexpr int kBoth = 2 * kWideRows > CK ? 2 * kWideRows : CK;
+                    const int rows = WIDE && hv.split ? kBoth : CK;
+                    const int target = ready_base + (min(k0 + rows, Pm1 + 1) + ready_rows - 1) / ready_rows;
                     if (ready_seen < target) {
                         if (!wait_word_at_least(ready, target, ctl.spin)) {
                             if (lane == 0) atomicOr(err, ERR_UPLOAD_TIMEOUT);
