@@ -420,6 +420,11 @@ int srg_bp_burst_device_noalloc(const srg_burst_desc *b, const srg_bp_options *o
  * sets it near there to run calls across the restart. */
 int srg_test_set_dropin_sequence(int device, int seq);
 
+/* Testing hook: 0: crossmul calls on the current device take cuFFT's
+ * transforms at every line length, as where the library's own do not fit the
+ * device; 1: back to the library's own. */
+int srg_test_crossmul_own(int use);
+
 /* Testing hook: the FP64 form's own steps of a term, as device code, on n (at
  * least 1) values: root[i] = sqrt(x[i]), quot[i] = x[i] / d[i], sn[i] and cs[i]
  * the sine and cosine of x[i].  Device pointers; enqueued on `stream`. */

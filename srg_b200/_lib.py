@@ -101,6 +101,7 @@ _SIGS = {
     "srg_bp_burst_device_gated": (C.c_int, [C.POINTER(BurstDesc), C.c_void_p, C.c_int, C.c_int,
                                             C.POINTER(Options), C.c_void_p]),
     "srg_test_set_dropin_sequence": (C.c_int, [C.c_int, C.c_int]),
+    "srg_test_crossmul_own": (C.c_int, [C.c_int]),
     "srg_test_fp64_steps_device": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int64] + [C.c_void_p] * 5),
     "srg_dropin_flush": (C.c_int, [C.c_int]),
     "srg_dropin_last_bytes": (C.c_int, [C.c_int, C.POINTER(C.c_longlong),

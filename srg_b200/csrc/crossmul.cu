@@ -28,8 +28,9 @@
 //     input sample) and crossmul_looks_kernel forms the looks: for nnn = 64 ..
 //     8,192 from odd_kernel, for nnn = 16,384 .. 65,536 from odd_cluster_kernel
 //     (a cluster of CTAs per line).
-//   * nnn < 64 and nnn > 65,536 (lines of up to 32 or over 65,536 samples):
-//     the transforms by cuFFT over padded rows.
+//   * nnn < 64 and nnn > 65,536 (lines of up to 32 or over 65,536 samples), and
+//     a plan whose CTA or cluster the device has no room for: the transforms by
+//     cuFFT over padded rows.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <cufft.h>
@@ -708,7 +709,8 @@ struct XmCtx {
     // per own plan: tables on the device, resident CTAs of the kernels
     DevBuf tab[kOwnPlans];
     int odd_ctas[kOwnPlans] = {}, stack_ctas[kOwnPlans] = {}, across_ctas[kOwnPlans] = {};
-    bool ready[kOwnPlans] = {};
+    bool ready[kOwnPlans] = {}, unfit[kOwnPlans] = {};  // unfit: does not fit the device's SMs
+    bool own_off = false;  // srg_test_crossmul_own
 };
 XmCtx g_xm[64];
 
@@ -741,9 +743,10 @@ void cluster_config(const OwnPlan &p, int grid, cudaStream_t st, cudaLaunchConfi
     cfg.numAttrs = p.cluster > 1 ? 1 : 0;
 }
 
-// Tables and launch limits of own plan `i` on the current device (made once).
+// Tables and launch limits of own plan `i` on the current device (made once),
+// or unfit[i].
 int ensure_plan(XmCtx &x, int i, int dev, cudaStream_t st) {
-    if (x.ready[i]) return SRG_OK;
+    if (x.ready[i] || x.unfit[i]) return SRG_OK;
     const OwnPlan &p = own_plans()[i];
     const std::vector<float2> t = p.tables();
     int rc = x.tab[i].ensure(sizeof(float2) * t.size());
@@ -758,13 +761,19 @@ int ensure_plan(XmCtx &x, int i, int dev, cudaStream_t st) {
             cudaLaunchConfig_t cfg{};
             cudaLaunchAttribute at{};
             cluster_config(p, sms * p.cluster, 0, cfg, at);
-            CKC(cudaOccupancyMaxActiveClusters(&ctas, fn, &cfg));
+            if (cudaOccupancyMaxActiveClusters(&ctas, fn, &cfg) != cudaSuccess) {
+                ctas = 0;  // a part of a device may be too small for the cluster
+                cudaGetLastError();
+            }
             ctas *= p.cluster;
         } else {
             CKC(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, fn, p.threads, p.smem));
             ctas *= sms;
         }
-        if (ctas < 1) return fail(SRG_E_UNSUPPORTED, "line transform of %d points does not fit an SM", p.nnn);
+        if (ctas < 1) {
+            x.unfit[i] = true;
+            return SRG_OK;
+        }
         (fn == p.odd ? x.odd_ctas : fn == p.stack ? x.stack_ctas : x.across_ctas)[i] = ctas;
     }
     CKC(cudaMemcpyAsync(x.tab[i].p, t.data(), sizeof(float2) * t.size(), cudaMemcpyHostToDevice, st));
@@ -839,9 +848,12 @@ int run_stack(const float *const *slcs, int n, long long ld, int na, int nlines,
     const int nnn = fft_length(na);
     const int nout_lines = nlines / looksdn, nout_cols = na / looksac;
     const int nl = nout_lines * looksdn;
-    const int own = own_plan_of(nnn);
+    int own = x.own_off ? -1 : own_plan_of(nnn);
     if (own >= 0) {
         if ((rc = ensure_plan(x, own, dev, st))) return rc;
+        if (x.unfit[own]) own = -1;  // cuFFT runs anywhere
+    }
+    if (own >= 0) {
         const OwnPlan &op = own_plans()[own];
         // (odd_stack_kernel takes scale / nnn / 2 as one factor, which must be a
         // normal number)
@@ -923,6 +935,15 @@ int run_stack(const float *const *slcs, int n, long long ld, int na, int nlines,
 }  // namespace
 
 extern "C" {
+
+int srg_test_crossmul_own(int use) {
+    int dev = 0;
+    CKC(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return fail(SRG_E_ARG, "device %d out of range", dev);
+    std::lock_guard<std::mutex> g(g_xm[dev].mu);
+    g_xm[dev].own_off = !use;
+    return SRG_OK;
+}
 
 int srg_crossmul_device(const float *slc1, const float *slc2, long long ld, int na, int nlines,
                         int looksac, int looksdn, float scale, int mask, float *igram, float *amp,
