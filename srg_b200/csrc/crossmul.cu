@@ -12,8 +12,10 @@
 // c = j looksac + k, i over the looksdn input lines of L (crossmul.f90:155-172);
 // amp likewise with (|u1|^2, |u2|^2), then (sqrt re, sqrt im) (:173); both
 // zeroed where |sum of the raw input over the look window| <= 1e-6 in either
-// image (crossmul.f90:112-125, 176-184).  Sums run in the reference's order
-// (reclaim, then down, then across) in FP32 as the reference's complex*8.
+// image (crossmul.f90:112-125, 176-184).  Sums run in FP32 as the reference's
+// complex*8 and in its order (reclaim, then down, then across), but that
+// odd_stack_kernel forms the reclaim's sum as one chain of FMAs, the odd
+// sample's products last.
 //
 // The transforms.  The forward and inverse transforms of steps 2-4 cancel at
 // the even upsampled samples: u[2n] = x_s[n] / 2 (x_s = in * scale).  The odd
@@ -366,7 +368,7 @@ odd_kernel(const __grid_constant__ OddArgs a, int nimg, long long ld, int na, in
 // through distributed shared memory and writes C outputs per n.  So one
 // exchange per line, of the line's size, and two CTAs of different lines share
 // an SM.  Bound by instruction issue (53 % of the cycles) and the latency of
-// its loads: two images of 16,504 x 6,646 samples take 3.7 ms, where padding,
+// its loads: two images of 16,504 x 6,646 samples take 3.75 ms, where padding,
 // cuFFT's transforms of 32,768 and 65,536 points and the spread took 12.0; a
 // cluster of two with 16,384 points each, alone on its SMs, took 5.3.  The
 // grid is what the chip holds of clusters at once (with more, the last ones

@@ -28,7 +28,9 @@
 // banks.
 //
 // Twiddles are exactly rounded entries of tables [r - 1][column], contiguous
-// over threads.
+// over threads; where a thread has several columns of pass 1 and the caller
+// keeps only the first ones' (Tw1: crossmul's 64 and 8,192 points), the others
+// are turned from them, which adds a rounding.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -114,8 +116,11 @@ __host__ __device__ constexpr int brev(int i) {
 // the ratio r of its sine and cosine (at most 1) and four for the sums scaled
 // by the larger of the two: six operations and two roundings per result,
 // against eight and three for the product and its sum and difference.  The
-// ratio's own rounding shows in long sums, though (range compression's error
-// against 64 bits 2.1e-7, 2.0e-7 without it): FUSED chooses.
+// ratio's own rounding shows in long sums, though: FUSED chooses.  Range
+// compression goes without it (error against 64 bits 2.0e-7, 2.1e-7 with it, both
+// before the gain below was taken out; 0.31 and 0.29 ms).  Crossmul takes it: its
+// odd samples' error is no larger for it (1.37e-7 at 4,096 points and 1.43e-7
+// without, the gain out, by the same operations on the CPU).
 template <bool INV, bool FUSED>
 __device__ __forceinline__ void butterfly(float2 &lo, float2 &hi, int m) {
     const float2 a = lo, b = hi;

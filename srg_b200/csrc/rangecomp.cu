@@ -95,10 +95,11 @@ __global__ void rc_out_kernel(const float2 *__restrict__ buf, int l0, int nlines
 // Bound by instruction issue (see fft_conv.cuh): 1,500 lines of 24,000 samples,
 // pulse of 3,371, take 0.31 ms (0.45 with self-sorting transforms of one segment
 // per 512-thread CTA), 700 lines of 29,001 with a pulse of 5,147 0.24 ms (0.58
-// with cuFFT).  With fused butterflies (Plan::FUSED) 0.29 ms and 5 % more error;
-// with the spectrum in shared memory and half the twiddles turned from the
-// others 0.30 and 10 % more; everything through L1 and two CTAs per SM 0.31, as two
-// halves of 4,096 points at 16 points per thread 0.42.
+// with cuFFT); error against 64 bits 1.8e-7 (2.0e-7 and 4.9e-7).  With fused
+// butterflies (Plan::FUSED) 0.29 ms and 5 % more error, before the transforms'
+// gain was taken out; with the spectrum in shared memory and half the twiddles
+// turned from the others 0.30 and 10 % more; everything through L1 and two CTAs per
+// SM 0.31, as two halves of 4,096 points at 16 points per thread 0.42.
 using Seg = fftc::Plan<8192, 32, 16, 16, 32, false>;
 constexpr int kOsM = Seg::M;                     // segment transform
 // Segments per line up to which the kernel is the faster path: one takes
